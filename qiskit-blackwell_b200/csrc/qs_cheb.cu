@@ -21,6 +21,7 @@ using namespace qs;
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kPauliThreads = 256;
 
 struct Acc { float s, c; };  // compensated sum: value = s + c
 
@@ -237,11 +238,18 @@ __global__ void k_chebp_fused(const PTerm* __restrict__ terms, int nterms, uint6
 //   * terms with x_t = 0 sum to a real diagonal D_i = sum_t c_t (-1)^{popc(i & z_t)},
 //     tabulated once per evolution (FP64 sums rounded to FP32, 4 B per
 //     amplitude), so the degree loop reads D_i instead of evaluating them;
-//   * the other terms are sorted by X mask and paired: both terms of a pair
-//     share one gather x[i ^ x] (e.g. X_a X_b and Y_a Y_b), and a lone term
-//     has a zero partner.  The sign (-1)^{popc(j & z)} is applied by flipping
-//     the sign bit of the weight.
-struct __align__(16) PPair { uint32_t x, z0, z1, pad; float w0r, w0i, w1r, w1i; };
+//   * every other weight w_t = c_t i^{|x_t & z_t|} is real or imaginary; terms
+//     of equal X mask and kind are paired (e.g. X_a X_b and Y_a Y_b) so that a
+//     pair shares its gather x[i ^ x], and a lone term has a zero partner.
+// The pairs come in four runs, real / imaginary weights by even / odd X masks.
+struct __align__(16) PMask {
+  uint32_t x;        // X mask
+  uint32_t z0, z1;   // Z masks without the bits a thread holds in registers
+  uint32_t pat;      // signs of those bits: byte 0 for z0, byte 1 for z1
+  float w0, w1;      // weights (real, or the factor of i)
+  float pad0, pad1;
+};
+struct PRuns { int r0, r1, i0, end; };  // [0,r0) real even, [r0,r1) real odd, [r1,i0) imaginary even, [i0,end) odd
 struct __align__(16) PDiag { uint64_t z; double c; };
 
 __global__ void k_chebp_diag(const PDiag* __restrict__ terms, int nterms, uint64_t n, float* __restrict__ D) {
@@ -258,66 +266,135 @@ __global__ void k_chebp_diag(const PDiag* __restrict__ terms, int nterms, uint64
 
 __device__ __forceinline__ float flip_if(float w, uint32_t sbit) { return __int_as_float(__float_as_int(w) ^ sbit); }
 
-__device__ __forceinline__ float2 hx_row_pairs(const PPair* __restrict__ st, int npairs, const float2* __restrict__ x,
-                                               const float* __restrict__ D, uint32_t i) {
-  float re = 0.f, im = 0.f;
-  if (D) {
-    const float d = D[i];
-    const float2 v = x[i];
-    re = d * v.x;
-    im = d * v.y;
+// One run of pairs on a thread's 2*M amplitudes (qubit 0, and qubits 6 and 7
+// for M = 4; v[m] is one 16-byte gather of two amplitudes, a warp's 32 lanes
+// covering 512 consecutive bytes of it).  The parity of the
+// index bits outside the registers is taken once for the 2*M amplitudes (POPC
+// runs at an eighth of the FP32 rate); inside them the sign is a bit of `pat`.
+// SWAP: the X mask has bit 0, so the two amplitudes of a gather trade places.
+template <int M, bool IMAG, bool SWAP>
+__device__ __forceinline__ void pauli_run(const PMask* __restrict__ sp, int b, int e, const float4* __restrict__ x4,
+                                          uint32_t t4, float2 (&acc)[2 * M]) {
+  auto add = [&](int r, float w, float vx, float vy) {
+    float2& a = acc[SWAP ? r ^ 1 : r];
+    if (IMAG) {
+      a.x = fmaf(-w, vy, a.x);
+      a.y = fmaf(w, vx, a.y);
+    } else {
+      a.x = fmaf(w, vx, a.x);
+      a.y = fmaf(w, vy, a.y);
+    }
+  };
+#pragma unroll 2
+  for (int k = b; k < e; ++k) {
+    const PMask P = sp[k];
+    const uint32_t j4 = t4 ^ (P.x >> 1);
+    float4 v[M];
+#pragma unroll
+    for (int m = 0; m < M; ++m) v[m] = x4[j4 ^ (uint32_t)(m << 5)];
+    const uint32_t j = j4 << 1;
+    const float w0 = flip_if(P.w0, (uint32_t)__popc(j & P.z0) << 31);
+    const float w1 = flip_if(P.w1, (uint32_t)__popc(j & P.z1) << 31);
+    if (P.pat == 0) {
+      const float w = w0 + w1;
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        add(2 * m, w, v[m].x, v[m].y);
+        add(2 * m + 1, w, v[m].z, v[m].w);
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < 2 * M; ++r) {
+        const float w = flip_if(w0, (P.pat << (31 - r)) & 0x80000000u) + flip_if(w1, (P.pat << (23 - r)) & 0x80000000u);
+        const float4 u = v[r >> 1];
+        add(r, w, (r & 1) ? u.z : u.x, (r & 1) ? u.w : u.y);
+      }
+    }
   }
-  for (int k = 0; k < npairs; ++k) {
-    const PPair P = st[k];
-    const uint32_t j = i ^ P.x;
-    const float2 v = x[j];
-    const uint32_t s0 = (uint32_t)(__popc(j & P.z0) & 1) << 31, s1 = (uint32_t)(__popc(j & P.z1) & 1) << 31;
-    const float wr = flip_if(P.w0r, s0) + flip_if(P.w1r, s1);
-    const float wi = flip_if(P.w0i, s0) + flip_if(P.w1i, s1);
-    re = fmaf(wr, v.x, fmaf(-wi, v.y, re));
-    im = fmaf(wr, v.y, fmaf(wi, v.x, im));
-  }
-  return make_float2(re, im);
 }
 
-__global__ void k_chebp_first_pairs(const PPair* __restrict__ pairs, int npairs, uint64_t n,
-                                    const float* __restrict__ D, const float2* __restrict__ x0,
-                                    float2* __restrict__ x1, float2* __restrict__ out, float scale, float2 c0,
-                                    float2 c1) {
+// One degree of the recurrence, x_{k+1} in place of x_{k-1} and accumulated
+// into out (FIRST: x_1 = scale H x_0 and out = c0 x_0 + c1 x_1).  S groups of a
+// CTA's threads share its amplitudes, each taking a part of every run; their
+// sums meet in shared memory in a fixed order.
+//
+// Bound by the gathers' L2 traffic and their issue slots.  22 qubits, 42 masks:
+// 73 us per degree; 176 us with one amplitude per thread, of which the two
+// POPCs of a pair (16 lanes per clock and SM) alone are 137.
+template <int M, int S, bool FIRST>
+__global__ void __launch_bounds__(kPauliThreads)
+    k_chebp_masks(const PMask* __restrict__ masks, PRuns R, uint32_t nthr, const float2* __restrict__ D,
+                  const float4* __restrict__ xk, float4* __restrict__ xprev, float4* __restrict__ out, float scale,
+                  float2 c0, float2 c) {
+  extern __shared__ __align__(16) PMask sm[];
+  constexpr int G = kPauliThreads / S;   // threads of a group, a multiple of 32
+  __shared__ float2 part[S > 1 ? S - 1 : 1][S > 1 ? 2 * M : 1][S > 1 ? G : 1];
+  // the table was copied before the first kernel of the evolution began, so
+  // it may be read before the kernel in front of this one has finished
+  for (int k = threadIdx.x; k < R.end; k += blockDim.x) sm[k] = masks[k];
   pdl_begin();
-  extern __shared__ PPair sp[];
-  for (int k = threadIdx.x; k < npairs; k += blockDim.x) sp[k] = pairs[k];
   __syncthreads();
-  for (uint64_t i = gtid(); i < n; i += gstride()) {
-    const float2 d = hx_row_pairs(sp, npairs, x0, D, (uint32_t)i);
-    const float2 t = make_float2(scale * d.x, scale * d.y);
-    x1[i] = t;
-    const float2 a0 = x0[i];
-    float2 a;
-    a.x = c0.x * a0.x - c0.y * a0.y;
-    a.y = c0.x * a0.y + c0.y * a0.x;
-    a.x = fmaf(c1.x, t.x, fmaf(-c1.y, t.y, a.x));
-    a.y = fmaf(c1.x, t.y, fmaf(c1.y, t.x, a.y));
-    out[i] = a;
+  const int s = threadIdx.x / G;
+  auto cut = [&](int b, int e, int k) { return b + (e - b) * k / S; };
+  const uint32_t g = blockIdx.x * (uint32_t)G + threadIdx.x % G;
+  const bool live = g < nthr;
+  const uint32_t t4 = (g >> 5) * (32u * M) + (g & 31u);
+  float2 acc[2 * M];
+#pragma unroll
+  for (int r = 0; r < 2 * M; ++r) acc[r] = make_float2(0.f, 0.f);
+  if (live) {
+    if (D && s == 0) {
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        const float2 d = D[t4 + 32 * m];
+        const float4 v = xk[t4 + 32 * m];
+        acc[2 * m] = make_float2(d.x * v.x, d.x * v.y);
+        acc[2 * m + 1] = make_float2(d.y * v.z, d.y * v.w);
+      }
+    }
+    pauli_run<M, false, false>(sm, cut(0, R.r0, s), cut(0, R.r0, s + 1), xk, t4, acc);
+    pauli_run<M, false, true>(sm, cut(R.r0, R.r1, s), cut(R.r0, R.r1, s + 1), xk, t4, acc);
+    pauli_run<M, true, false>(sm, cut(R.r1, R.i0, s), cut(R.r1, R.i0, s + 1), xk, t4, acc);
+    pauli_run<M, true, true>(sm, cut(R.i0, R.end, s), cut(R.i0, R.end, s + 1), xk, t4, acc);
   }
-}
-
-__global__ void k_chebp_fused_pairs(const PPair* __restrict__ pairs, int npairs, uint64_t n,
-                                    const float* __restrict__ D, const float2* __restrict__ xk,
-                                    float2* __restrict__ xprev, float2* __restrict__ out, float two_scale,
-                                    float2 c) {
-  pdl_begin();
-  extern __shared__ PPair sp[];
-  for (int k = threadIdx.x; k < npairs; k += blockDim.x) sp[k] = pairs[k];
-  __syncthreads();
-  for (uint64_t i = gtid(); i < n; i += gstride()) {
-    const float2 d = hx_row_pairs(sp, npairs, xk, D, (uint32_t)i);
-    const float2 p = xprev[i];
-    const float2 t = make_float2(fmaf(two_scale, d.x, -p.x), fmaf(two_scale, d.y, -p.y));
+  if (S > 1) {
+    if (s > 0) {
+#pragma unroll
+      for (int r = 0; r < 2 * M; ++r) part[s - 1][r][threadIdx.x % G] = acc[r];
+    }
+    __syncthreads();
+    if (s > 0) return;
+    for (int q = 0; q < S - 1; ++q) {
+#pragma unroll
+      for (int r = 0; r < 2 * M; ++r) {
+        const float2 v = part[q][r][threadIdx.x];
+        acc[r].x += v.x;
+        acc[r].y += v.y;
+      }
+    }
+  }
+  if (!live) return;
+#pragma unroll
+  for (int m = 0; m < M; ++m) {
+    const uint32_t i = t4 + 32 * m;
+    const float2 d0 = acc[2 * m], d1 = acc[2 * m + 1];
+    float4 t, a;
+    if (FIRST) {
+      t = make_float4(scale * d0.x, scale * d0.y, scale * d1.x, scale * d1.y);
+      const float4 v = xk[i];
+      a = make_float4(c0.x * v.x - c0.y * v.y, c0.x * v.y + c0.y * v.x, c0.x * v.z - c0.y * v.w,
+                      c0.x * v.w + c0.y * v.z);
+    } else {
+      const float4 p = xprev[i];
+      t = make_float4(fmaf(scale, d0.x, -p.x), fmaf(scale, d0.y, -p.y), fmaf(scale, d1.x, -p.z),
+                      fmaf(scale, d1.y, -p.w));
+      a = out[i];
+    }
     xprev[i] = t;
-    float2 a = out[i];
     a.x = fmaf(c.x, t.x, fmaf(-c.y, t.y, a.x));
     a.y = fmaf(c.x, t.y, fmaf(c.y, t.x, a.y));
+    a.z = fmaf(c.x, t.z, fmaf(-c.y, t.w, a.z));
+    a.w = fmaf(c.x, t.w, fmaf(c.y, t.z, a.w));
     out[i] = a;
   }
 }
@@ -461,34 +538,55 @@ int qs_cheb_evolve_pauli(qs_handle_t h, int n, const void* psi, void* out, const
   auto C = [&](int k) { return make_float2((float)coeffs[2 * k], (float)coeffs[2 * k + 1]); };
   const float two_scale = (float)(2.0 * scale);
   if (n <= 32) {
-    // diagonal terms and X-mask pairs (see PPair)
+    // Amplitudes per thread and groups per CTA.  Below 2^16 amplitudes a degree
+    // is the latency of the mask loop, so two amplitudes per thread and the
+    // masks over 8 groups (13 qubits, 84 terms, t = 2: 450 us; 594 in one
+    // group); to 2^18 eight amplitudes and 4 groups keep the SMs filled (18
+    // qubits 918 us; 1024 in one group); above, one group (22 qubits 73 us per
+    // degree; 110 in 4 groups, 94 with two amplitudes per thread).
+    const int M = n < 16 ? 1 : 4, S = n < 16 ? 8 : n < 19 ? 4 : 1;
+    const uint32_t regs = M == 4 ? 0xC1u : 0x01u;   // the index bits inside a thread
     std::vector<PDiag> dg;
     std::vector<int> off;
     for (int k = 0; k < nterms; ++k) {
       if (xm[k] == 0) dg.push_back(PDiag{zm[k], coefs[k]});
       else off.push_back(k);
     }
-    std::stable_sort(off.begin(), off.end(), [&](int a, int b) { return xm[a] < xm[b]; });
-    std::vector<PPair> pr;
-    for (size_t u = 0; u < off.size();) {
-      const PTerm& A = T[off[u]];
-      PPair P{(uint32_t)A.x, (uint32_t)A.z, 0u, 0u, A.wr, A.wi, 0.f, 0.f};
-      if (u + 1 < off.size() && xm[off[u + 1]] == xm[off[u]]) {
-        const PTerm& B = T[off[u + 1]];
-        P.z1 = (uint32_t)B.z;
-        P.w1r = B.wr;
-        P.w1i = B.wi;
-        u += 2;
-      } else {
-        u += 1;
+    auto run_of = [&](int k) { return 2 * (__builtin_popcountll(xm[k] & zm[k]) & 1) + (int)(xm[k] & 1); };
+    std::stable_sort(off.begin(), off.end(), [&](int a, int b) {
+      return run_of(a) != run_of(b) ? run_of(a) < run_of(b) : xm[a] < xm[b];
+    });
+    // signs over a thread's 2*M source amplitudes: bit 2m + e for the gather
+    // that output m reads, whose own register bits are m ^ (those of x)
+    auto pattern = [&](uint64_t x, uint64_t z) {
+      uint32_t pat = 0;
+      for (int r = 0; r < 2 * M; ++r) {
+        const uint64_t j = (uint64_t)(r & 1) | (((uint64_t)(r >> 1) << 6) ^ (x & regs & ~1ull));
+        pat |= (uint32_t)(__builtin_popcountll(j & z & regs) & 1) << r;
       }
-      pr.push_back(P);
+      return pat;
+    };
+    std::vector<PMask> pm;
+    int ends[4] = {0, 0, 0, 0};
+    for (size_t u = 0; u < off.size();) {
+      const int a = off[u], run = run_of(a);
+      auto weight = [&](int k) { return run < 2 ? T[k].wr : T[k].wi; };
+      PMask P{(uint32_t)xm[a], (uint32_t)zm[a] & ~regs, 0u, pattern(xm[a], zm[a]), weight(a), 0.f, 0.f, 0.f};
+      ++u;
+      if (u < off.size() && xm[off[u]] == xm[a] && run_of(off[u]) == run) {
+        const int b = off[u++];
+        P.z1 = (uint32_t)zm[b] & ~regs;
+        P.pat |= pattern(xm[b], zm[b]) << 8;
+        P.w1 = weight(b);
+      }
+      pm.push_back(P);
+      for (int r = run; r < 4; ++r) ends[r] = (int)pm.size();
     }
-    const size_t pbytes = sizeof(PPair) * pr.size(), dbytes = sizeof(PDiag) * dg.size();
+    const size_t pbytes = sizeof(PMask) * pm.size(), dbytes = sizeof(PDiag) * dg.size();
     char* dmem = (char*)h->scratch_get(std::max<size_t>(16, pbytes + dbytes));
-    const PPair* dP = (const PPair*)dmem;
+    const PMask* dP = (const PMask*)dmem;
     const PDiag* dD = (const PDiag*)(dmem + pbytes);
-    if (pbytes) QS_CUDA(cudaMemcpyAsync(dmem, pr.data(), pbytes, cudaMemcpyHostToDevice, h->stream));
+    if (pbytes) QS_CUDA(cudaMemcpyAsync(dmem, pm.data(), pbytes, cudaMemcpyHostToDevice, h->stream));
     if (dbytes) QS_CUDA(cudaMemcpyAsync(dmem + pbytes, dg.data(), dbytes, cudaMemcpyHostToDevice, h->stream));
     float* D = nullptr;
     if (!dg.empty()) {
@@ -498,15 +596,20 @@ int qs_cheb_evolve_pauli(qs_handle_t h, int n, const void* psi, void* out, const
     }
     try {
       QS_CUDA(cudaMemcpyAsync(x0, psi, sizeof(float2) * N, cudaMemcpyDeviceToDevice, h->stream));
-      const unsigned grid = (unsigned)qs_blocks_for(h, N, kThreads, 8);
-      const int np = (int)pr.size();
-      qs_launch_pdl(h, k_chebp_first_pairs, dim3(grid), dim3(kThreads), pbytes, dP, np, N, D, x0, x1, (float2*)out,
-                                                                 (float)scale, C(0), C(1));
-      qs_after_launch(h, "k_chebp_first_pairs");
+      const uint32_t nthr = (uint32_t)(N / (2 * M));
+      const uint32_t per = (uint32_t)(kPauliThreads / S);
+      const dim3 grid((unsigned)((nthr + per - 1) / per));
+      const PRuns R{ends[0], ends[1], ends[2], ends[3]};
+      auto step = [&](auto kern, const float2* xk, float2* xp, float s, float2 c0, float2 c) {
+        qs_launch_pdl(h, kern, grid, dim3(kPauliThreads), pbytes, dP, R, nthr, (const float2*)D, (const float4*)xk,
+                      (float4*)xp, (float4*)out, s, c0, c);
+        qs_after_launch(h, "k_chebp_masks");
+      };
+      auto first = M == 1 ? k_chebp_masks<1, 8, true> : S == 4 ? k_chebp_masks<4, 4, true> : k_chebp_masks<4, 1, true>;
+      auto next = M == 1 ? k_chebp_masks<1, 8, false> : S == 4 ? k_chebp_masks<4, 4, false> : k_chebp_masks<4, 1, false>;
+      step(first, x0, x1, (float)scale, C(0), C(1));
       for (int k = 2; k <= K; ++k) {
-        qs_launch_pdl(h, k_chebp_fused_pairs, dim3(grid), dim3(kThreads), pbytes, dP, np, N, D, x1, x0, (float2*)out,
-                                                                   two_scale, C(k));
-        qs_after_launch(h, "k_chebp_fused_pairs");
+        step(next, x1, x0, two_scale, C(0), C(k));
         std::swap(x0, x1);
       }
     } catch (...) {
