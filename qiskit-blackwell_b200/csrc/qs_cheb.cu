@@ -1,7 +1,10 @@
 // qs_cheb.cu — CSR SpMV and the Chebyshev recurrence for exp(-iHt)|psi>.
 //
-// Rows are processed by V-lane sub-warps (V = 4..32, picked from the mean row
-// length) so that the col_idx/values streams are read coalesced.  Each lane
+// Rows are processed by V-lane sub-warps (V = 1..32, picked from the mean row
+// length and the number of rows).  A 20-qubit Hamiltonian of 30 entries per row
+// takes 104 us per degree with V = 4 (4.3 TB/s of its 12 nnz + 44 N bytes) and
+// 322 us with a warp per row, whose gathers used 8 bytes of each 32-byte sector
+// and whose merge cost 150 instructions per row.  Each lane
 // accumulates its entries with error-free products and TwoSum (a compensated
 // "Kahan" row sum); lanes are combined in a fixed shuffle order, also
 // compensated, so results are deterministic.
@@ -55,13 +58,30 @@ __device__ __forceinline__ float2 row_dot(const int32_t* __restrict__ rp, const 
   int32_t b = 0, e = 0;
   if (r >= 0) { b = rp[r]; e = rp[r + 1]; }
   Acc re{0.f, 0.f}, im{0.f, 0.f};
-  for (int32_t j = b + lane; j < e; j += V) {
-    const float2 v = val[j];
-    const float2 xj = x[ci[j]];
-    acc_add_prod(re, v.x, xj.x);
-    acc_add_prod(re, -v.y, xj.y);
-    acc_add_prod(im, v.x, xj.y);
-    acc_add_prod(im, v.y, xj.x);
+  // kAhead entries of a lane in flight: their columns and values, then the
+  // gathers, then the sums (in the row's order).  More of them help the wide
+  // rows and only add predicated work to the short ones.
+  constexpr int kAhead = V <= 4 ? 2 : 4;
+  for (int32_t j = b + lane; j < e; j += V * kAhead) {
+    int32_t col[kAhead];
+    float2 v[kAhead], xj[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const bool in = j + u * V < e;
+      col[u] = in ? ci[j + u * V] : -1;
+      v[u] = in ? val[j + u * V] : make_float2(0.f, 0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (col[u] >= 0) xj[u] = x[col[u]];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      if (col[u] < 0) break;
+      acc_add_prod(re, v[u].x, xj[u].x);
+      acc_add_prod(re, -v[u].y, xj[u].y);
+      acc_add_prod(im, v[u].x, xj[u].y);
+      acc_add_prod(im, v[u].y, xj[u].x);
+    }
   }
   re = acc_reduce<V>(re);
   im = acc_reduce<V>(im);
@@ -406,14 +426,24 @@ int pick_V(int64_t nrows, const int32_t* rp_dev, qs_context* h) {
   QS_CUDA(cudaMemcpyAsync(&ends[1], rp_dev + nrows, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
   QS_CUDA(cudaStreamSynchronize(h->stream));
   const double mean = nrows > 0 ? double(ends[1] - ends[0]) / double(nrows) : 1.0;
-  if (mean <= 6) return 4;
-  if (mean <= 12) return 8;
-  if (mean <= 28) return 16;
-  return 32;
+  // Few lanes per row: a warp then covers rows whose columns lie together, so
+  // a gather's 32-byte sectors are used whole, and fewer lanes are merged by
+  // shuffles.  Measured (64 M entries, us for V = 1 / 2 / 4 / 8 / 16 / 32):
+  // 5 per row 120 / 136 / 181 / 292 / 576 / 1149, 20 per row 126 / 107 / 106 /
+  // 132 / 194 / 318, 200 per row 178 / 118 / 118 / 97 / 105 / 124, 2000 per row
+  // 1189 / 623 / 338 / 128 / 120 / 107.
+  int V = mean <= 10 ? 1 : mean <= 16 ? 2 : mean <= 80 ? 4 : mean <= 250 ? 8 : mean <= 1000 ? 16 : 32;
+  // A matrix with few rows is bound by the latency of a lane's entries: more
+  // lanes until there are threads for every SM (13 qubits, 29 per row: V = 4
+  // 549 us an evolution, V = 8 500).
+  while (nrows * V < (1 << 16) && V < 32 && 2 * V <= mean) V *= 2;
+  return V;
 }
 
 #define DISPATCH_V(V, KERN, GRID, ...)                                            \
   switch (V) {                                                                   \
+    case 1: qs_launch_pdl(h, KERN<1>, dim3(GRID), dim3(kThreads), 0, __VA_ARGS__); break;       \
+    case 2: qs_launch_pdl(h, KERN<2>, dim3(GRID), dim3(kThreads), 0, __VA_ARGS__); break;       \
     case 4: qs_launch_pdl(h, KERN<4>, dim3(GRID), dim3(kThreads), 0, __VA_ARGS__); break;       \
     case 8: qs_launch_pdl(h, KERN<8>, dim3(GRID), dim3(kThreads), 0, __VA_ARGS__); break;       \
     case 16: qs_launch_pdl(h, KERN<16>, dim3(GRID), dim3(kThreads), 0, __VA_ARGS__); break;     \
