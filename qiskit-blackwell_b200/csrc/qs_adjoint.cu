@@ -30,8 +30,8 @@
 
 using namespace qs;
 
-void* qs_upload_terms(qs_context* h, size_t offset, int n, const uint64_t* x, const uint64_t* z, const double* c,
-                      int nterms);
+void qs_pauli_apply(qs_context* h, const float2* in, float2* out, uint64_t vstride, int nb, int n, const uint64_t* x,
+                    const uint64_t* z, const double* c, int nterms);
 
 namespace {
 
@@ -177,31 +177,6 @@ __global__ void k_adj_final(const double* __restrict__ partial, int nbx, double*
   if (threadIdx.x == 0) {
     double* o = out + (uint64_t)b * ostride + idx;
     *o = add ? (*o + acc) : acc;
-  }
-}
-
-// k_pauli_apply equivalent per vector: lam = H psi (defined in qs_reduce.cu
-// for a single state; re-stated here for the strided batch layout).
-struct TermL { uint64_t x, z; double wr, wi; };
-__global__ void k_adj_hpsi(float2* __restrict__ base, uint64_t vstride, uint64_t n, const TermL* __restrict__ terms,
-                           int nterms) {
-  extern __shared__ TermL st[];
-  for (int k = threadIdx.x; k < nterms; k += blockDim.x) st[k] = terms[k];
-  __syncthreads();
-  const int b = blockIdx.y;
-  const float2* psi = base + (uint64_t)b * vstride;
-  float2* lam = base + (uint64_t)b * vstride + (vstride / 3);
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    double re = 0.0, im = 0.0;
-    for (int k = 0; k < nterms; ++k) {
-      const TermL T = st[k];
-      const uint64_t j = i ^ T.x;
-      const float2 v = psi[j];
-      const double sg = (__popcll(j & T.z) & 1) ? -1.0 : 1.0;
-      re += sg * (T.wr * v.x - T.wi * v.y);
-      im += sg * (T.wr * v.y + T.wi * v.x);
-    }
-    lam[i] = make_float2((float)re, (float)im);
   }
 }
 
@@ -702,11 +677,8 @@ extern "C" int qs_adjoint_gradient(qs_handle_t h, int n, const qs_op* ops, int n
   }
 
   // ---- lam = H psi, E = Re<psi|lam>
-  TermL* dT = (TermL*)qs_upload_terms(h, 0, n, xm, zm, coefs, nterms);
   {
-    dim3 grid((unsigned)std::min<uint64_t>((N + kThreads - 1) / kThreads, 64), nb);
-    k_adj_hpsi<<<grid, kThreads, sizeof(TermL) * nterms, h->stream>>>((float2*)work, vstride, N, dT, nterms);
-    qs_after_launch(h, "k_adj_hpsi");
+    qs_pauli_apply(h, (const float2*)work, (float2*)work + N, vstride, nb, n, xm, zm, coefs, nterms);
     k_adj_dot<<<dim3(sd.nbx, nb), kThreads, 0, h->stream>>>((const float2*)work, vstride, N, sd.per, d_part);
     qs_after_launch(h, "k_adj_dot");
     k_adj_final<<<nb, kThreads, 0, h->stream>>>(d_part, sd.nbx, d_energy, 1, 0, 0);

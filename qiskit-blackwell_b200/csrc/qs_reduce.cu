@@ -11,6 +11,7 @@
 #include "qs_common.cuh"
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <map>
 #include <mutex>
 
@@ -20,6 +21,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kMaxBlocks = 1024;
+constexpr int kPauliBlocks = 888;   // 148 SMs x 2 resident CTAs x 3
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -492,79 +494,317 @@ __global__ void k_sample_b(const float2* __restrict__ base, const SampleDesc* __
 }
 
 // ---------------------------------------------------- Pauli-sum terms ----
-// Term t: coefficient w_t = coef_t * i^{popc(x_t & z_t)} (complex), x_t, z_t.
-// (P psi)[i] = i^{|x&z|} (-1)^{popc((i^x) & z)} psi[i ^ x].
-struct Term { uint64_t x, z; double wr, wi; };
+// (P_t psi)[i] = i^{|x&z|} (-1)^{popc(j & z)} psi[j], j = i ^ x, for the string
+// with masks x, z.  A term's weight is therefore real or i times a real c_t.
+// Terms are grouped by X mask: row i of a mask has the weight
+// W_x(j) = sum_t c_t (-1)^{popc(j & z_t)} (FP64) on the one gathered psi[j].
+//
+// A thread holds 2*M amplitudes (qubit 0, and qubits 6 and 7 for M = 4), a
+// gather being 16 bytes of which a warp reads 512 in a row.  The parity of the
+// index bits outside the registers is taken once per term and thread, the rest
+// of the sign is a bit of `pat`.  The masks come in four runs: real / imaginary
+// weights, each with even then odd X masks (SWAP: the two amplitudes of a
+// gather trade places).
+template <class U>
+struct alignas(8) PauliMask {
+  U x;
+  U hbit, hval;             // expectation: threads with (index & hbit) != hval skip the mask
+  int32_t t0, tu, t1;       // terms [t0, t1), those before tu of equal sign in all registers
+};
+template <class U>
+struct alignas(8) PauliTerm {
+  double c;
+  U z;                      // without the bits held in registers
+  uint32_t pat;             // signs over the registers: bit 2m + e
+};
+struct PauliRuns { int r0, r1, i0, end, terms; };  // real even, real odd, imaginary even, imaginary odd
 
-__device__ __forceinline__ void term_apply(const Term& T, uint64_t i, const float2* __restrict__ s, double& re,
-                                           double& im) {
-  const uint64_t j = i ^ T.x;
-  const float2 b = s[j];
-  const double sg = (__popcll(j & T.z) & 1) ? -1.0 : 1.0;
-  re += sg * (T.wr * b.x - T.wi * b.y);
-  im += sg * (T.wr * b.y + T.wi * b.x);
+__device__ __forceinline__ uint32_t parity_bit(uint32_t v) { return (uint32_t)__popc(v) << 31; }
+__device__ __forceinline__ uint32_t parity_bit(uint64_t v) { return (uint32_t)__popcll(v) << 31; }
+__device__ __forceinline__ double flip_if(double v, uint32_t sign) {
+  return __hiloint2double(__double2hiint(v) ^ (int)sign, __double2loint(v));
 }
 
-// <psi|H|psi> partials: sum_i Re(conj(psi_i) (H psi)_i)
-__global__ void k_pauli_expect(const float2* __restrict__ s, uint64_t n, const Term* __restrict__ terms, int nterms,
-                               uint64_t per, double* __restrict__ partial) {
-  pdl_begin();
-  extern __shared__ Term st[];
-  for (int k = threadIdx.x; k < nterms; k += blockDim.x) st[k] = terms[k];
+// The weights of one mask over a thread's amplitudes; returns whether they are
+// all w[0].
+template <int M, class U>
+__device__ __forceinline__ bool mask_weights(const PauliMask<U>& P, const PauliTerm<U>* __restrict__ st, U j,
+                                             double (&w)[2 * M]) {
+  double w0 = 0.0;
+  for (int t = P.t0; t < P.tu; ++t) w0 += flip_if(st[t].c, parity_bit((U)(j & st[t].z)));
+  w[0] = w0;
+  if (P.tu == P.t1) return true;
+#pragma unroll
+  for (int r = 1; r < 2 * M; ++r) w[r] = w0;
+  for (int t = P.tu; t < P.t1; ++t) {
+    const double c = flip_if(st[t].c, parity_bit((U)(j & st[t].z)));
+    const uint32_t pat = st[t].pat;
+#pragma unroll
+    for (int r = 0; r < 2 * M; ++r) w[r] += flip_if(c, (pat << (31 - r)) & 0x80000000u);
+  }
+  return false;
+}
+
+template <int M, bool IMAG, bool SWAP, class U>
+__device__ __forceinline__ void pauli_rows(const PauliMask<U>* __restrict__ sm, const PauliTerm<U>* __restrict__ st,
+                                           int b, int e, const float4* __restrict__ x4, U t4, double2 (&acc)[2 * M]) {
+  for (int k = b; k < e; ++k) {
+    const PauliMask<U> P = sm[k];
+    const U j4 = t4 ^ (P.x >> 1);
+    float4 v[M];
+#pragma unroll
+    for (int m = 0; m < M; ++m) v[m] = x4[j4 ^ (U)(m << 5)];
+    double w[2 * M];
+    const bool same = mask_weights<M, U>(P, st, (U)(j4 << 1), w);
+    auto add = [&](int r, double wr) {
+      const double vx = (r & 1) ? v[r >> 1].z : v[r >> 1].x, vy = (r & 1) ? v[r >> 1].w : v[r >> 1].y;
+      double2& a = acc[SWAP ? r ^ 1 : r];
+      if (IMAG) {
+        a.x = fma(-wr, vy, a.x);
+        a.y = fma(wr, vx, a.y);
+      } else {
+        a.x = fma(wr, vx, a.x);
+        a.y = fma(wr, vy, a.y);
+      }
+    };
+    if (same) {
+#pragma unroll
+      for (int r = 0; r < 2 * M; ++r) add(r, w[0]);
+    } else {
+#pragma unroll
+      for (int r = 0; r < 2 * M; ++r) add(r, w[r]);
+    }
+  }
+}
+
+// Re sum_i conj(psi_i) W psi_{i^x} over the rows the masks select.
+template <int M, bool IMAG, bool SWAP, class U>
+__device__ __forceinline__ void pauli_dot(const PauliMask<U>* __restrict__ sm, const PauliTerm<U>* __restrict__ st,
+                                          int b, int e, const float4* __restrict__ x4, U t4,
+                                          const double2 (&a)[2 * M], double& acc) {
+  for (int k = b; k < e; ++k) {
+    const PauliMask<U> P = sm[k];
+    if (((t4 << 1) & P.hbit) != P.hval) continue;
+    const U j4 = t4 ^ (P.x >> 1);
+    float4 v[M];
+#pragma unroll
+    for (int m = 0; m < M; ++m) v[m] = x4[j4 ^ (U)(m << 5)];
+    double w[2 * M];
+    const bool same = mask_weights<M, U>(P, st, (U)(j4 << 1), w);
+    double s[4] = {0.0, 0.0, 0.0, 0.0};   // chains of their own
+#pragma unroll
+    for (int r = 0; r < 2 * M; ++r) {
+      const double2 p = a[SWAP ? r ^ 1 : r];
+      const double vx = (r & 1) ? v[r >> 1].z : v[r >> 1].x, vy = (r & 1) ? v[r >> 1].w : v[r >> 1].y;
+      if (same) {
+        s[r & 1] = fma(IMAG ? p.y : p.x, vx, s[r & 1]);
+        s[2 + (r & 1)] = fma(IMAG ? -p.x : p.y, vy, s[2 + (r & 1)]);
+      } else {
+        s[r & 3] = fma(w[r], IMAG ? fma(p.y, vx, -p.x * vy) : fma(p.x, vx, p.y * vy), s[r & 3]);
+      }
+    }
+    acc = fma(same ? w[0] : 1.0, (s[0] + s[1]) + (s[2] + s[3]), acc);
+  }
+}
+
+template <int M>
+constexpr uint32_t pauli_regs() { return M == 4 ? 0xC1u : M == 2 ? 0x41u : 0x01u; }
+
+// The table of a Pauli sum, masks then terms, in shared memory.
+template <class U>
+__device__ __forceinline__ const PauliTerm<U>* pauli_stage(const uint32_t* __restrict__ table, PauliRuns R,
+                                                           PauliMask<U>* sm) {
+  const uint32_t words = (uint32_t)((sizeof(PauliMask<U>) * R.end + sizeof(PauliTerm<U>) * R.terms) / 4);
+  uint32_t* d = reinterpret_cast<uint32_t*>(sm);
+  for (uint32_t k = threadIdx.x; k < words; k += blockDim.x) d[k] = table[k];
   __syncthreads();
-  const uint64_t b0 = (uint64_t)blockIdx.x * per;
-  const uint64_t e = min(b0 + per, n);
+  return reinterpret_cast<const PauliTerm<U>*>(sm + R.end);
+}
+
+// out = H psi (complex64), accumulated in FP64 per amplitude; blockIdx.y is
+// the vector.  S groups of a CTA's threads share its amplitudes, each taking a
+// part of every run of masks.
+//
+// Bound by the FP32-to-FP64 conversions of the gathered amplitudes (16 lanes
+// per clock and SM, two per mask and amplitude).  8 vectors of 20 qubits, 256
+// random terms: 848 us; 3436 with one amplitude per thread and term (two
+// 32-bit POPCs and six FP64 operations each).
+template <int M, int S, class U>
+__global__ void __launch_bounds__(kThreads, 3)
+    k_pauli_apply(const float2* __restrict__ in, float2* __restrict__ out, uint64_t vstride,
+                  const uint32_t* __restrict__ table, PauliRuns R, U nthr) {
+  pdl_begin();
+  extern __shared__ __align__(16) unsigned char pauli_smem[];
+  constexpr int G = kThreads / S;
+  __shared__ double2 part[S > 1 ? S - 1 : 1][S > 1 ? 2 * M : 1][S > 1 ? G : 1];
+  auto* sm = reinterpret_cast<PauliMask<U>*>(pauli_smem);
+  const PauliTerm<U>* st = pauli_stage(table, R, sm);
+  const float4* x4 = reinterpret_cast<const float4*>(in + blockIdx.y * vstride);
+  float4* o4 = reinterpret_cast<float4*>(out + blockIdx.y * vstride);
+  const int s = threadIdx.x / G;
+  auto cut = [&](int b, int e, int k) { return b + (e - b) * k / S; };
+  const U g = (U)blockIdx.x * G + threadIdx.x % G;
+  const bool has = g < nthr;
+  const U t4 = (g >> 5) * (U)(32 * M) + (g & 31);
+  double2 acc[2 * M];
+#pragma unroll
+  for (int r = 0; r < 2 * M; ++r) acc[r] = make_double2(0.0, 0.0);
+  if (has) {
+    pauli_rows<M, false, false, U>(sm, st, cut(0, R.r0, s), cut(0, R.r0, s + 1), x4, t4, acc);
+    pauli_rows<M, false, true, U>(sm, st, cut(R.r0, R.r1, s), cut(R.r0, R.r1, s + 1), x4, t4, acc);
+    pauli_rows<M, true, false, U>(sm, st, cut(R.r1, R.i0, s), cut(R.r1, R.i0, s + 1), x4, t4, acc);
+    pauli_rows<M, true, true, U>(sm, st, cut(R.i0, R.end, s), cut(R.i0, R.end, s + 1), x4, t4, acc);
+  }
+  if (S > 1) {
+    if (s > 0) {
+#pragma unroll
+      for (int r = 0; r < 2 * M; ++r) part[s - 1][r][threadIdx.x % G] = acc[r];
+    }
+    __syncthreads();
+    if (s > 0) return;
+    for (int q = 0; q < S - 1; ++q) {
+#pragma unroll
+      for (int r = 0; r < 2 * M; ++r) {
+        const double2 v = part[q][r][threadIdx.x];
+        acc[r].x += v.x;
+        acc[r].y += v.y;
+      }
+    }
+  }
+  if (!has) return;
+#pragma unroll
+  for (int m = 0; m < M; ++m)
+    o4[t4 + (U)(32 * m)] = make_float4((float)acc[2 * m].x, (float)acc[2 * m].y, (float)acc[2 * m + 1].x,
+                                       (float)acc[2 * m + 1].y);
+}
+
+// <psi|H|psi> partials, one per CTA.  Rows i and i ^ x of a mask contribute
+// the same real part, so where x has a bit that a whole warp shares, one of
+// the two is evaluated and the weights are doubled on the host.
+//
+// Bound as k_pauli_apply by conversions: 24 qubits, 64 random terms
+// 460 us; 1535 with one amplitude per thread and term.
+template <int M, int S, class U>
+__global__ void __launch_bounds__(kThreads, 3)
+    k_pauli_expect(const float2* __restrict__ psi, const uint32_t* __restrict__ table, PauliRuns R, U nthr,
+                   double* __restrict__ partial) {
+  pdl_begin();
+  extern __shared__ __align__(16) unsigned char pauli_smem[];
+  constexpr int G = kThreads / S;
+  auto* sm = reinterpret_cast<PauliMask<U>*>(pauli_smem);
+  const PauliTerm<U>* st = pauli_stage(table, R, sm);
+  const float4* x4 = reinterpret_cast<const float4*>(psi);
+  const int s = threadIdx.x / G;
+  auto cut = [&](int b, int e, int k) { return b + (e - b) * k / S; };
   double acc = 0.0;
-  for (uint64_t i = b0 + threadIdx.x; i < e; i += blockDim.x) {
-    double re = 0.0, im = 0.0;
-    for (int k = 0; k < nterms; ++k) term_apply(st[k], i, s, re, im);
-    const float2 a = s[i];
-    acc += (double)a.x * re + (double)a.y * im;
+  for (U g = (U)blockIdx.x * G + threadIdx.x % G; g < nthr; g += (U)gridDim.x * G) {
+    const U t4 = (g >> 5) * (U)(32 * M) + (g & 31);
+    double2 a[2 * M];
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      const float4 v = x4[t4 + (U)(32 * m)];
+      a[2 * m] = make_double2(v.x, v.y);
+      a[2 * m + 1] = make_double2(v.z, v.w);
+    }
+    pauli_dot<M, false, false, U>(sm, st, cut(0, R.r0, s), cut(0, R.r0, s + 1), x4, t4, a, acc);
+    pauli_dot<M, false, true, U>(sm, st, cut(R.r0, R.r1, s), cut(R.r0, R.r1, s + 1), x4, t4, a, acc);
+    pauli_dot<M, true, false, U>(sm, st, cut(R.r1, R.i0, s), cut(R.r1, R.i0, s + 1), x4, t4, a, acc);
+    pauli_dot<M, true, true, U>(sm, st, cut(R.i0, R.end, s), cut(R.i0, R.end, s + 1), x4, t4, a, acc);
   }
   acc = block_sum(acc);
   if (threadIdx.x == 0) partial[blockIdx.x] = acc;
 }
 
-// out = H psi (complex64), accumulated in FP64 per amplitude.
-__global__ void k_pauli_apply(const float2* __restrict__ s, float2* __restrict__ out, uint64_t n,
-                              const Term* __restrict__ terms, int nterms) {
-  pdl_begin();
-  extern __shared__ Term st[];
-  for (int k = threadIdx.x; k < nterms; k += blockDim.x) st[k] = terms[k];
-  __syncthreads();
-  for (uint64_t i = gtid(); i < n; i += gstride()) {
-    double re = 0.0, im = 0.0;
-    for (int k = 0; k < nterms; ++k) term_apply(st[k], i, s, re, im);
-    out[i] = make_float2((float)re, (float)im);
+struct PauliUpload { const uint32_t* table; PauliRuns runs; size_t bytes; };
+
+// Builds the table in scratch after `offset` bytes.  `regs`: the index bits a
+// thread holds in registers; `halve`: choose one of the rows i and i ^ x.
+template <class U>
+PauliUpload pauli_upload(qs_context* h, size_t offset, int n, const uint64_t* x, const uint64_t* z, const double* c,
+                         int nterms, uint32_t regs, bool halve) {
+  QS_CHECK_ARG(nterms >= 1, "need at least one Pauli term");
+  QS_CHECK_ARG(x && z && c, "term pointers are null");
+  const uint64_t lim = (1ull << n) - 1ull;
+  std::vector<int> order(nterms);
+  for (int k = 0; k < nterms; ++k) {
+    QS_CHECK_ARG((x[k] & ~lim) == 0 && (z[k] & ~lim) == 0, "Pauli mask has bits beyond n_qubits");
+    order[k] = k;
   }
+  // real weight: |x & z| even; run 2 * imaginary + odd X mask
+  auto run_of = [&](int k) { return 2 * (__builtin_popcountll(x[k] & z[k]) & 1) + (int)(x[k] & 1); };
+  // signs of the amplitudes that a thread reads for its outputs: bit 2m + e
+  auto pattern = [&](int k) {
+    uint32_t pat = 0;
+    for (int r = 0; r < 8; ++r) {
+      const uint64_t j = (uint64_t)(r & 1) | (((uint64_t)(r >> 1) << 6) ^ (x[k] & regs & ~1ull));
+      pat |= (uint32_t)(__builtin_popcountll(j & z[k] & regs) & 1) << r;
+    }
+    return pat & (regs == 0x01u ? 0x3u : regs == 0x41u ? 0xFu : 0xFFu);
+  };
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+    if (run_of(a) != run_of(b)) return run_of(a) < run_of(b);
+    if (x[a] != x[b]) return x[a] < x[b];
+    return (pattern(a) == 0) > (pattern(b) == 0);
+  });
+  std::vector<PauliMask<U>> masks;
+  std::vector<PauliTerm<U>> terms;
+  int ends[4] = {0, 0, 0, 0};
+  for (int u = 0; u < nterms;) {
+    const int a = order[u], run = run_of(a);
+    PauliMask<U> P{(U)x[a], 0, 0, u, u, u};
+    const uint64_t warp_bits = x[a] & ~(uint64_t)(regs | 0x3Eu);
+    if (halve && warp_bits) {
+      P.hbit = (U)(warp_bits & (~warp_bits + 1));
+      P.hval = (masks.size() & 1) ? P.hbit : 0;   // alternate, so that no CTA has all the work
+    }
+    const double scale = P.hbit ? 2.0 : 1.0;
+    for (; u < nterms && run_of(order[u]) == run && x[order[u]] == x[a]; ++u) {
+      const int k = order[u];
+      const int ny = __builtin_popcountll(x[k] & z[k]) & 3;   // i^ny = +-1 or +-i
+      const uint32_t pat = pattern(k);
+      terms.push_back(PauliTerm<U>{(ny >= 2 ? -c[k] : c[k]) * scale, (U)z[k] & ~(U)regs, pat});
+      if (pat == 0) P.tu = u + 1;
+    }
+    P.t1 = u;
+    masks.push_back(P);
+    for (int r = run; r < 4; ++r) ends[r] = (int)masks.size();
+  }
+  const size_t mb = sizeof(PauliMask<U>) * masks.size(), tb = sizeof(PauliTerm<U>) * terms.size();
+  std::vector<char> host(mb + tb);
+  std::memcpy(host.data(), masks.data(), mb);
+  std::memcpy(host.data() + mb, terms.data(), tb);
+  char* d = (char*)h->scratch_get(offset + mb + tb) + offset;
+  // From pageable memory the copy returns once it has been staged, so the
+  // host vector may go out of scope afterwards.
+  QS_CUDA(cudaMemcpyAsync(d, host.data(), mb + tb, cudaMemcpyHostToDevice, h->stream));
+  return {(const uint32_t*)d, {ends[0], ends[1], ends[2], ends[3], nterms}, mb + tb};
+}
+
+template <int M, int S, class U>
+void pauli_apply(qs_context* h, const float2* in, float2* out, uint64_t vstride, int nb, int n, const uint64_t* x,
+                 const uint64_t* z, const double* c, int nterms) {
+  const PauliUpload T = pauli_upload<U>(h, 0, n, x, z, c, nterms, pauli_regs<M>(), false);
+  const uint64_t nthr = (1ull << n) / (2 * M), per = kThreads / S;
+  if (T.bytes > 32 * 1024)   // 48 KiB without the attribute, static arrays included
+    QS_CUDA(cudaFuncSetAttribute(k_pauli_apply<M, S, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T.bytes));
+  qs_launch_pdl(h, k_pauli_apply<M, S, U>, dim3((unsigned)((nthr + per - 1) / per), nb), dim3(kThreads), T.bytes, in, out,
+                vstride, T.table, T.runs, (U)nthr);
+  qs_after_launch(h, "k_pauli_apply");
 }
 
 }  // namespace
 
-// Builds the device term table (records of {x, z, w_re, w_im}) in scratch
-// after `offset` bytes.
-void* qs_upload_terms(qs_context* h, size_t offset, int n, const uint64_t* x, const uint64_t* z, const double* c,
-                      int nterms);
-
-void* qs_upload_terms(qs_context* h, size_t offset, int n, const uint64_t* x, const uint64_t* z, const double* c,
-                      int nterms) {
-  QS_CHECK_ARG(nterms >= 1, "need at least one Pauli term");
-  QS_CHECK_ARG(x && z && c, "term pointers are null");
-  const uint64_t lim = n >= 64 ? ~0ull : ((1ull << n) - 1ull);
-  std::vector<Term> T(nterms);
-  for (int k = 0; k < nterms; ++k) {
-    QS_CHECK_ARG((x[k] & ~lim) == 0 && (z[k] & ~lim) == 0, "Pauli mask has bits beyond n_qubits");
-    const int ny = __builtin_popcountll(x[k] & z[k]) & 3;
-    // i^ny
-    static const double pr[4] = {1, 0, -1, 0}, pi[4] = {0, 1, 0, -1};
-    T[k] = Term{x[k], z[k], c[k] * pr[ny], c[k] * pi[ny]};
-  }
-  char* base = (char*)h->scratch_get(offset + sizeof(Term) * nterms);
-  Term* d = (Term*)(base + offset);
-  // From pageable memory the copy returns once T has been staged, so the
-  // host vector may go out of scope afterwards.
-  QS_CUDA(cudaMemcpyAsync(d, T.data(), sizeof(Term) * nterms, cudaMemcpyHostToDevice, h->stream));
-  return d;
+// out_b = H in_b (complex64, FP64 sums) for nb vectors `vstride` amplitudes
+// apart; 16-byte aligned, not aliased.
+void qs_pauli_apply(qs_context* h, const float2* in, float2* out, uint64_t vstride, int nb, int n, const uint64_t* x,
+                    const uint64_t* z, const double* c, int nterms) {
+  // Eight amplitudes per thread once they fill the SMs; below, two, and the
+  // masks over 8 groups of threads: with 64 terms an expectation value takes
+  // 45 us less at 12 qubits than with eight amplitudes, as much at 18, and 27
+  // us more at 19.
+  if (n > 32) pauli_apply<4, 1, uint64_t>(h, in, out, vstride, nb, n, x, z, c, nterms);
+  else if (n >= 8 && ((uint64_t)nb << n) >= (1ull << 18)) pauli_apply<4, 1, uint32_t>(h, in, out, vstride, nb, n, x, z, c, nterms);
+  else pauli_apply<1, 8, uint32_t>(h, in, out, vstride, nb, n, x, z, c, nterms);
 }
 
 namespace {
@@ -581,6 +821,21 @@ void reduce_to(qs_context* h, F f, uint64_t items, double* d_out, int mode, doub
 // scratch layout for reductions: [0, 16) two doubles out; [64, ...) partials
 double* red_out(qs_context* h) { return (double*)h->scratch_get(64 + 8 * kMaxBlocks); }
 double* red_part(qs_context* h) { return (double*)((char*)h->scratch_get(64 + 8 * kMaxBlocks) + 64); }
+
+// Leaves <psi|H|psi> in red_out.  The slicing depends on n only.
+template <int M, int S, class U>
+void pauli_expect(qs_context* h, const float2* psi, int n, const uint64_t* x, const uint64_t* z, const double* c,
+                  int nterms) {
+  const PauliUpload T = pauli_upload<U>(h, 64 + 8 * kMaxBlocks, n, x, z, c, nterms, pauli_regs<M>(), true);
+  const uint64_t nthr = (1ull << n) / (2 * M), per = kThreads / S;
+  const int nb = (int)std::min<uint64_t>((nthr + per - 1) / per, kPauliBlocks);
+  if (T.bytes > 32 * 1024)   // 48 KiB without the attribute, static arrays included
+    QS_CUDA(cudaFuncSetAttribute(k_pauli_expect<M, S, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T.bytes));
+  qs_launch_pdl(h, k_pauli_expect<M, S, U>, dim3(nb), dim3(kThreads), T.bytes, psi, T.table, T.runs, (U)nthr, red_part(h));
+  qs_after_launch(h, "k_pauli_expect");
+  qs_launch_pdl(h, k_final, dim3(1), dim3(1024), 0, red_part(h), nb, red_out(h), 0);
+  qs_after_launch(h, "k_final");
+}
 
 double fetch_scalar(qs_context* h, const double* d) {
   double* pin = h->pinned_get(64);
@@ -679,17 +934,10 @@ int qs_expect_pauli_sum(qs_handle_t h, const void* state, int n, const uint64_t*
   qs_check_state(state, n);
   QS_CHECK_ARG(out != nullptr, "out is null");
   QS_CHECK_ARG(nterms >= 1 && nterms <= 1024, "n_terms must be in [1, 1024]");
-  const size_t toff = 64 + 8 * kMaxBlocks;
-  Term* dT = (Term*)qs_upload_terms(h, toff, n, x, z, c, nterms);
+  if (n > 32) pauli_expect<4, 1, uint64_t>(h, (const float2*)state, n, x, z, c, nterms);
+  else if (n >= 18) pauli_expect<4, 1, uint32_t>(h, (const float2*)state, n, x, z, c, nterms);
+  else pauli_expect<1, 8, uint32_t>(h, (const float2*)state, n, x, z, c, nterms);
   double* o = red_out(h);
-  double* part = red_part(h);
-  const uint64_t N = 1ull << n;
-  Slicing sl = slice(N);
-  qs_launch_pdl(h, k_pauli_expect, dim3(sl.nb), dim3(kThreads), sizeof(Term) * nterms, (const float2*)state, N, dT, nterms, sl.per,
-                                                                        part);
-  qs_after_launch(h, "k_pauli_expect");
-  qs_launch_pdl(h, k_final, dim3(1), dim3(1024), 0, part, sl.nb, o, 0);
-  qs_after_launch(h, "k_final");
   *out = fetch_scalar(h, o);
   QS_API_END(h)
 }
@@ -702,11 +950,7 @@ int qs_apply_pauli_sum(qs_handle_t h, const void* psi, void* out, int n, const u
   qs_check_state(out, n);
   QS_CHECK_ARG(psi != out, "out must not alias psi");
   QS_CHECK_ARG(nterms >= 1 && nterms <= 1024, "n_terms must be in [1, 1024]");
-  Term* dT = (Term*)qs_upload_terms(h, 0, n, x, z, c, nterms);
-  const uint64_t N = 1ull << n;
-  qs_launch_pdl(h, k_pauli_apply, dim3(qs_blocks_for(h, N, kThreads)), dim3(kThreads), sizeof(Term) * nterms, 
-      (const float2*)psi, (float2*)out, N, dT, nterms);
-  qs_after_launch(h, "k_pauli_apply");
+  qs_pauli_apply(h, (const float2*)psi, (float2*)out, 0, 1, n, x, z, c, nterms);
   QS_API_END(h)
 }
 
