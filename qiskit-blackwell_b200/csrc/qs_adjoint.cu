@@ -7,17 +7,12 @@
 //                  psi <- U_l^dag psi,  lam <- U_l^dag lam.
 // (2 Re<lam| dU/dtheta |psi_{l-1}> = 2 Re(-i/2 <lam|G U psi_{l-1}>) = Im<lam|G|psi_l>.)
 //
-// The forward pass uses the batch planner (all parameter vectors in one set
-// of tile-pass launches).  The reverse sweep is cut into tile passes too:
-// consecutive (reversed) gates whose targets fit one tile of T qubits (the
-// low qubits plus those the gates touch; controls may lie anywhere) run in one
-// launch over all tiles of all parameter vectors.  A CTA stages the tile of
-// both psi and lam in shared memory, applies every gate's U^dag there and, for
-// each parameter gate, writes its FP64 partial of Im<lam|G|psi> (taken before
-// the gate is undone); a final kernel sums the partials in a fixed order
-// (deterministic).  So psi and lam cross HBM once per pass instead of once per
-// gate.  QSIM_ADJ_PASSES=0 selects the older one-launch-per-gate sweep (kept
-// for comparison; same arithmetic per gate, different summation order).
+// Both sweeps are cut into tile passes (below): psi, in the reverse sweep psi
+// and lambda, cross HBM once per pass instead of once per gate, and CTAs apply
+// the gates of a pass to a tile in shared memory.  The FP64 partial sums of
+// <lambda|P|psi> are reduced in a fixed order (deterministic).
+// QSIM_ADJ_PASSES=0, or very many partials, selects the older sweep (a
+// batch-planned forward, then one launch per gate; kept for comparison).
 // There is no reference counterpart (ROADMAP.md:173-175 lists adjoint
 // differentiation as future work).
 #include "qs_api.h"
@@ -26,7 +21,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
-#include <set>
+#include <type_traits>
 
 using namespace qs;
 
@@ -180,203 +175,492 @@ __global__ void k_adj_final(const double* __restrict__ partial, int nbx, double*
   }
 }
 
-// ------------------------------------------------ reverse-sweep passes ----
-enum AdjKind : int32_t { AG_1Q = 1, AG_MCX = 2, AG_PHASE = 3, AG_U2 = 4 };
+// ------------------------------------------------------ tile passes ----
+// A pass is a list of steps on a tile of 2^T amplitudes staged in shared
+// memory.  A tile bit k (position) has an address column: amplitude i lies at
+// the XOR of the columns of its set bits and a constant.  So X and CNOT move
+// nothing: they change the constant or add one column to another (a control
+// outside the tile adds a constant in the tiles where it is 1).  The first
+// columns also spread the tile over the banks.
+//
+// Kinds of step:
+//   block  three positions (forward: four) whose pending 1Q gates are fused into
+//          one 2x2 matrix each (k_adj_prepare).  A thread
+//          holds the amplitudes over those bits in registers; in the reverse
+//          sweep psi and lambda share a matrix, packed for two-lane FMAs.
+//          All parameter gates of a position's run are rotations about axes
+//          that the rest of the run turns, so their gradients are combinations
+//          of three sums, Im<lambda|P|psi> for P = X, Y, Z, taken before the run
+//          is undone.
+//   MCX (two or more controls), phase, U2: one sweep of the tile.
+//   store  the last: the tile goes back in the order of its columns.
+enum AdjKind : int32_t { AG_BLOCK = 0, AG_MCX, AG_PHASE, AG_U2, AG_STORE };
 
-struct AdjGate {
+constexpr int kAdjTileBits = 12;
+constexpr int kAdjLowQubits = 4;
+constexpr int kAdjOut = 8;
+
+struct alignas(16) AdjStep {
   int32_t kind;
-  int32_t p0, p1;     // tile positions of the target(s); U2: p0 = matrix bit 0
-  int32_t gkind;      // 1Q parameter gate generator: 1 X, 2 Y, 3 Z; 0 none
-  int32_t slot;       // partial-sum slot of a parameter gate, else -1
-  int32_t mat;        // 1Q: op index into the per-(op, vector) U^dag table; U2: Mat4 index
-  int32_t neg;        // phase: negate instead of multiplying
-  int32_t pad;
-  uint64_t cmask;     // MCX controls / phase qubits, as a global index mask
-  float2 ph;          // phase factor (already conjugated)
-  float2 pad2;
+  int32_t mat;               // U2: Mat4 index
+  uint16_t col[kAdjTileBits];  // block: columns of the thread index; others: of the tile bits (all in bytes)
+  uint16_t v[4];             // block: columns of the register bits
+  uint16_t c, nout;
+  int32_t slot[3];           // first of a run's three sums, or -1
+  uint32_t out[kAdjOut];     // controls outside the tile: qubit << 16 | constant
+  uint64_t cmask;            // MCX controls / phase qubits, as a global index mask
+  float2 ph;                 // phase factor (already conjugated)
+  uint8_t p0, p1;            // tile positions of the targets; U2: p0 = matrix bit 0
+  uint8_t neg;               // phase: negate instead of multiplying
+  uint8_t gates;             // block: bit j set where position j has a matrix
+  uint32_t pad[5];
 };
+static_assert(sizeof(AdjStep) == 128, "eight 16-byte loads");
 
 struct PassArg {
-  int32_t S[16];      // tile positions (global qubits), ascending
-  int32_t T;
-  int32_t gb, ge;     // gate range of the pass
-  int32_t nslots;     // parameter-gate slots of the whole sweep
+  int32_t S[kAdjTileBits];  // tile positions (global qubits), ascending
+  int32_t T, bits;    // tile bits, and those of them that exist (n < T)
+  int32_t gb, ge;     // steps of the pass
+  int32_t nslots;     // sums of the whole sweep
   int32_t from_zero;  // forward: the tile starts as |0..0> instead of being loaded
-  int32_t pad[3];
 };
-
-__device__ __forceinline__ double block_sum_fixed(double v, double* red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) red[w] = v;
-  __syncthreads();
-  double t = 0.0;
-  if (threadIdx.x == 0)
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) t += red[k];
-  __syncthreads();
-  return t;  // valid on thread 0
-}
 
 __device__ __forceinline__ float2 conjf2(float2 a) { return make_float2(a.x, -a.y); }
 
-// One pass: CTA (tile, vector b).  Reverse (FWD false): psi and lam tiles
-// staged, every gate's U^dag applied to both, parameter-gate partials
-// written.  Forward (FWD true): psi only, every gate's U applied (the
-// conjugate transpose of the stored U^dag), from |0..0> when P.from_zero.
-// Shared memory: psi tile, lam tile (reverse only; 2^T float2 each), then the
-// 2 x 128 dep tables.
-template <bool FWD>
-__global__ void __launch_bounds__(kThreads) k_adj_pass(float2* __restrict__ base, uint64_t vstride, PassArg P,
-                                                      const AdjGate* __restrict__ gates,
-                                                      const Mat2* __restrict__ udag, int nb,
-                                                      const Mat4* __restrict__ u2, double* __restrict__ partial) {
-  extern __shared__ __align__(16) unsigned char adj_smem[];
-  const int T = P.T;
-  const uint32_t NT = 1u << T;
-  float2* sp = reinterpret_cast<float2*>(adj_smem);
-  float2* sl = FWD ? sp : sp + NT;
-  uint64_t* dep_lo = reinterpret_cast<uint64_t*>(sp + (FWD ? NT : 2 * NT));
-  uint64_t* dep_hi = dep_lo + 128;
-  __shared__ double red[kThreads / 32];
-  const int b = blockIdx.y;
-  const uint64_t tile = blockIdx.x, ntiles = gridDim.x;
-  float2* psi = base + (uint64_t)b * vstride;
-  float2* lam = psi + (vstride / 3);
-  for (int e = threadIdx.x; e < 256; e += blockDim.x) {
-    const int part = e >> 7, x = e & 127;
-    uint64_t d = 0;
-    for (int k = 0; k < 7; ++k) {
-      const int kk = part * 7 + k;
-      if (kk < T && ((x >> k) & 1)) d |= 1ull << P.S[kk];
-    }
-    if (part == 0) dep_lo[x] = d; else dep_hi[x] = d;
-  }
-  uint64_t gbase = tile;
-  for (int k = 0; k < T; ++k) gbase = insert_zero(gbase, P.S[k]);
-  __syncthreads();
-  auto gidx = [&](uint32_t i) { return gbase | dep_lo[i & 127] | dep_hi[i >> 7]; };
-  if (FWD && P.from_zero) {
-    const bool first = gbase == 0;
-    for (uint32_t i = threadIdx.x; i < NT; i += blockDim.x) sp[i] = make_float2(first && i == 0 ? 1.f : 0.f, 0.f);
+// The column of position k before any CNOT, in elements.  Its low four bits
+// choose the banks: powers of a primitive element of GF(16), so that four
+// neighbours span them all, also after chains of CNOTs (sums of neighbours are
+// such powers again).
+__host__ __device__ constexpr uint32_t adj_first_col(int k) {
+  return (1u << k) | (uint32_t)((0xE7A5BC638421ull >> (4 * k)) & 15);
+}
+
+// Sums v[0..N) over the warp; returns the index of the total that this lane's
+// v[0] then holds, -1 if none.  Each round passes half of the values on, so
+// nine cost 12 exchanges instead of 45.
+template <int N, int O>
+__device__ __forceinline__ void warp_totals_round(double* v, int lane, int& base, int& end) {
+  constexpr int H = (N + 1) / 2;
+  const bool up = lane & O;
+  if (N == 1) {
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], O);
   } else {
-    for (uint32_t i = threadIdx.x; i < NT; i += blockDim.x) {
-      const uint64_t g = gidx(i);
-      sp[i] = psi[g];
-      if (!FWD) sl[i] = lam[g];
+#pragma unroll
+    for (int k = 0; k < H; ++k) {
+      const double hi = k + H < N ? v[k + H] : 0.0;
+      const double keep = up ? hi : v[k], send = up ? v[k] : hi;
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, O);
     }
+    if (up) base += H; else end = min(end, base + H);
   }
-  __syncthreads();
-  for (int gi = P.gb; gi < P.ge; ++gi) {
-    const AdjGate G = gates[gi];
-    if (G.kind == AG_1Q) {
-      Mat2 U = udag[(uint64_t)G.mat * nb + b];
-      if (FWD) {
-        const float2 u1 = U.g[1];
-        U.g[0] = conjf2(U.g[0]);
-        U.g[1] = conjf2(U.g[2]);
-        U.g[2] = conjf2(u1);
-        U.g[3] = conjf2(U.g[3]);
-      }
-      const int p = G.p0;
-      double acc = 0.0;
-      for (uint32_t c = threadIdx.x; c < (NT >> 1); c += blockDim.x) {
-        const uint32_t i0 = (uint32_t)insert_zero(c, p), i1 = i0 | (1u << p);
-        const float2 a0 = sp[i0], a1 = sp[i1];
-        if (FWD) {
-          sp[i0] = cfma2(U.g[0], a0, U.g[1], a1);
-          sp[i1] = cfma2(U.g[2], a0, U.g[3], a1);
-          continue;
-        }
-        const float2 l0 = sl[i0], l1 = sl[i1];
-        if (G.gkind) {
-          float2 g0, g1;
-          if (G.gkind == 1) { g0 = a1; g1 = a0; }
-          else if (G.gkind == 2) { g0 = make_float2(a1.y, -a1.x); g1 = make_float2(-a0.y, a0.x); }
-          else { g0 = a0; g1 = make_float2(-a1.x, -a1.y); }
-          acc += (double)l0.x * g0.y - (double)l0.y * g0.x + (double)l1.x * g1.y - (double)l1.y * g1.x;
-        }
-        sp[i0] = cfma2(U.g[0], a0, U.g[1], a1);
-        sp[i1] = cfma2(U.g[2], a0, U.g[3], a1);
-        sl[i0] = cfma2(U.g[0], l0, U.g[1], l1);
-        sl[i1] = cfma2(U.g[2], l0, U.g[3], l1);
-      }
-      if (!FWD && G.slot >= 0) {
-        const double t = block_sum_fixed(acc, red);
-        if (threadIdx.x == 0) partial[((uint64_t)b * P.nslots + G.slot) * ntiles + tile] = t;
-      }
-    } else if (G.kind == AG_MCX) {
-      const int p = G.p0;
-      for (uint32_t c = threadIdx.x; c < (NT >> 1); c += blockDim.x) {
-        const uint32_t i0 = (uint32_t)insert_zero(c, p), i1 = i0 | (1u << p);
-        if ((gidx(i0) & G.cmask) != G.cmask) continue;
-        const float2 a0 = sp[i0];
-        sp[i0] = sp[i1];
-        sp[i1] = a0;
-        if (!FWD) {
-          const float2 l0 = sl[i0];
-          sl[i0] = sl[i1];
-          sl[i1] = l0;
-        }
-      }
-    } else if (G.kind == AG_PHASE) {
-      const float2 ph = FWD ? conjf2(G.ph) : G.ph;
-      for (uint32_t i = threadIdx.x; i < NT; i += blockDim.x) {
-        if ((gidx(i) & G.cmask) != G.cmask) continue;
-        const float2 a = sp[i];
-        sp[i] = G.neg ? make_float2(-a.x, -a.y) : cmul_comp(a, ph);
-        if (!FWD) {
-          const float2 l = sl[i];
-          sl[i] = G.neg ? make_float2(-l.x, -l.y) : cmul_comp(l, ph);
-        }
-      }
-    } else {  // AG_U2
-      Mat4 U = u2[G.mat];
-      if (FWD) {
-        const Mat4 D = U;
+  if constexpr (O > 1) warp_totals_round<H, O / 2>(v, lane, base, end);
+}
+template <int N>
+__device__ __forceinline__ int warp_totals(double (&v)[N], int lane) {
+  int base = 0, end = N;
+  warp_totals_round<N, 16>(v, lane, base, end);
+  return base < end ? base : -1;
+}
+
+// U on the pairs of register bit J of eight packed amplitudes.
+template <int J>
+__device__ __forceinline__ void adj_gate(float2 (&re)[8], float2 (&im)[8], const float4* __restrict__ U) {
+  // row by row, each entry twice for the two lanes: (x0, y0), (-y0, x1), (y1, -y1)
+  auto lo = [](float4 q) { return make_float2(q.x, q.y); };
+  auto hi = [](float4 q) { return make_float2(q.z, q.w); };
+  const float4 a0 = U[0], a1 = U[1], a2 = U[2], b0 = U[3], b1 = U[4], b2 = U[5];
+  const float2 g0x = lo(a0), g0y = hi(a0), m0y = lo(a1), g1x = hi(a1), g1y = lo(a2), m1y = hi(a2);
+  const float2 g2x = lo(b0), g2y = hi(b0), m2y = lo(b1), g3x = hi(b1), g3y = lo(b2), m3y = hi(b2);
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) U.g[4 * r + c] = conjf2(D.g[4 * c + r]);
-      }
-      const int lo = min(G.p0, G.p1), hi = max(G.p0, G.p1);
-      const uint32_t s0 = 1u << G.p0, s1 = 1u << G.p1;
-      for (uint32_t c = threadIdx.x; c < (NT >> 2); c += blockDim.x) {
-        const uint32_t i = (uint32_t)insert_zero(insert_zero(c, lo), hi);
-        float2* vs[2] = {sp, sl};
-#pragma unroll
-        for (int v = 0; v < (FWD ? 1 : 2); ++v) {
-          float2* x = vs[v];
-          const float2 a0 = x[i], a1 = x[i | s0], a2 = x[i | s1], a3 = x[i | s0 | s1];
-          x[i] = cfma4(U.g + 0, a0, a1, a2, a3);
-          x[i | s0] = cfma4(U.g + 4, a0, a1, a2, a3);
-          x[i | s1] = cfma4(U.g + 8, a0, a1, a2, a3);
-          x[i | s0 | s1] = cfma4(U.g + 12, a0, a1, a2, a3);
-        }
-      }
-    }
-    __syncthreads();
-  }
-  for (uint32_t i = threadIdx.x; i < NT; i += blockDim.x) {
-    const uint64_t g = gidx(i);
-    psi[g] = sp[i];
-    if (!FWD) lam[g] = sl[i];
+  for (int q = 0; q < 4; ++q) {
+    const int i = ((q >> J) << (J + 1)) | (q & ((1 << J) - 1)), k = i | (1 << J);
+    const float2 r0 = re[i], i0 = im[i], r1 = re[k], i1 = im[k];
+    re[i] = __ffma2_rn(m1y, i1, __ffma2_rn(g1x, r1, __ffma2_rn(m0y, i0, __fmul2_rn(g0x, r0))));
+    im[i] = __ffma2_rn(g1y, r1, __ffma2_rn(g1x, i1, __ffma2_rn(g0y, r0, __fmul2_rn(g0x, i0))));
+    re[k] = __ffma2_rn(m3y, i1, __ffma2_rn(g3x, r1, __ffma2_rn(m2y, i0, __fmul2_rn(g2x, r0))));
+    im[k] = __ffma2_rn(g3y, r1, __ffma2_rn(g3x, i1, __ffma2_rn(g2y, r0, __fmul2_rn(g2x, i0))));
   }
 }
 
-// grads[b][param_of[s]] += sum over tiles of partial[b][s][tile], slots in
-// order, tiles in order (deterministic).
-__global__ void k_adj_slots(const double* __restrict__ partial, int nslots, uint64_t ntiles,
-                            const int32_t* __restrict__ param_of, double* __restrict__ grads, int nparams) {
-  __shared__ double red[kThreads / 32];
-  const int b = blockIdx.x;
-  for (int sidx = 0; sidx < nslots; ++sidx) {
-    double acc = 0.0;
-    const double* p = partial + ((uint64_t)b * nslots + sidx) * ntiles;
-    for (uint64_t t = threadIdx.x; t < ntiles; t += blockDim.x) acc += p[t];
-    const double t = block_sum_fixed(acc, red);
-    if (threadIdx.x == 0) grads[(uint64_t)b * nparams + param_of[sidx]] += t;
+// U on the pairs of register bit J of 16 amplitudes.
+template <int J>
+__device__ __forceinline__ void adj_gate(float2 (&a)[16], const float4* __restrict__ U) {
+  const float4 A = U[0], B = U[1];
+  const float2 g0 = make_float2(A.x, A.y), g1 = make_float2(A.z, A.w), g2 = make_float2(B.x, B.y),
+               g3 = make_float2(B.z, B.w);
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int i = ((q >> J) << (J + 1)) | (q & ((1 << J) - 1)), k = i | (1 << J);
+    const float2 a0 = a[i], a1 = a[k];
+    a[i] = cfma2(g0, a0, g1, a1);
+    a[k] = cfma2(g2, a0, g3, a1);
   }
+}
+
+// Im<lambda|P|psi> for P = X, Y, Z on register bit J, in FP64.
+template <int J>
+__device__ __forceinline__ void adj_sums(const double2 (&a)[8], const double2 (&l)[8], double* s) {
+  double t[2][3] = {{s[0], s[1], s[2]}, {0.0, 0.0, 0.0}};   // two chains per sum
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int i = ((q >> J) << (J + 1)) | (q & ((1 << J) - 1)), k = i | (1 << J);
+    const double2 a0 = a[i], a1 = a[k], l0 = l[i], l1 = l[k];
+    double* u = t[q & 1];
+    u[0] = fma(l0.x, a1.y, fma(-l0.y, a1.x, fma(l1.x, a0.y, fma(-l1.y, a0.x, u[0]))));
+    u[1] = fma(-l0.x, a1.x, fma(-l0.y, a1.y, fma(l1.x, a0.x, fma(l1.y, a0.y, u[1]))));
+    u[2] = fma(l0.x, a0.y, fma(-l0.y, a0.x, fma(-l1.x, a1.y, fma(l1.y, a1.x, u[2]))));
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) s[k] = t[0][k] + t[1][k];
+}
+
+// One pass: CTA (tile, vector b).  Reverse (FWD false): psi and lambda, each
+// element of the tile (psi.re, lambda.re, psi.im, lambda.im).  Forward: psi
+// only, from |0..0> when P.from_zero.
+//
+// Bound by issue and FP64/conversion latency (16 warps per SM): a reverse block
+// of three runs is 16 shared loads and stores, 32 conversions, 144 FP64 and 192
+// packed FMAs per eight amplitudes; a forward block of four, 512 FMAs per 16.
+// 8 vectors of 20 qubits, 200 parameters: 8 reverse passes of 226 us and 7
+// forward ones of 102 us on average; one sweep of the tile per gate, with eight
+// conversions per pair and parameter gate, took 9 x 493 and 8 x 237 us.
+template <bool FWD>
+__global__ void __launch_bounds__(kThreads, FWD ? 3 : 2)
+    k_adj_pass(float2* __restrict__ base, uint64_t vstride, PassArg P, const AdjStep* __restrict__ steps,
+               const float4* __restrict__ mats, int nb, const Mat4* __restrict__ u2, double* __restrict__ partial) {
+  using Elem = typename std::conditional<FWD, float2, float4>::type;
+  extern __shared__ __align__(16) unsigned char adj_smem[];
+  constexpr uint32_t kElem = sizeof(Elem);
+  constexpr int kRegs = FWD ? 4 : 3, kMat = FWD ? 2 : 6;   // a staged matrix in 16-byte words
+  auto el = [&](uint32_t byte) -> Elem& { return *reinterpret_cast<Elem*>(adj_smem + byte); };
+  __shared__ uint64_t dep_lo[64], dep_hi[32];   // global index of a pair of amplitudes (tile bits 1-6, 7-11)
+  __shared__ uint16_t map_lo[64], map_hi[64];
+  __shared__ __align__(16) uint4 next[2][8 + kRegs * kMat];   // a step and its matrices (see adj_gate)
+  __shared__ double red[2][kThreads / 32][9];
+  const int T = P.T, tid = threadIdx.x, lane = tid & 31;
+  const uint32_t NT = 1u << T;
+  const int b = blockIdx.y;
+  const uint64_t tile = blockIdx.x, ntiles = gridDim.x;
+  float4* psi = reinterpret_cast<float4*>(base + (uint64_t)b * vstride);
+  float4* lam = reinterpret_cast<float4*>(base + (uint64_t)b * vstride + vstride / 3);
+  if (tid < 96) {
+    const int first = tid < 64 ? 1 : 7, x = tid < 64 ? tid : tid - 64;
+    uint64_t d = 0;
+    for (int k = 0; first + k < P.bits && k < 6; ++k)
+      if ((x >> k) & 1) d |= 1ull << P.S[first + k];
+    if (tid < 64) dep_lo[x] = d; else dep_hi[x] = d;
+  }
+  constexpr int kChunks = 8 + 2 * kRegs;   // by one thread each, all of warp 0
+  auto step_chunk = [&](int s) -> uint4 {
+    if (tid < 8) return reinterpret_cast<const uint4*>(steps + s)[tid];
+    const int j = (tid - 8) >> 1;
+    return reinterpret_cast<const uint4*>(mats)[(((uint64_t)s * 4 + j) * nb + b) * 2 + (tid & 1)];
+  };
+  auto step_put = [&](int buf, uint4 d) {
+    if (FWD || tid < 8) { next[buf][tid] = d; return; }
+    uint4* m = next[buf] + 8 + 3 * (tid - 8);
+    const uint32_t neg = 0x80000000u;
+    m[0] = make_uint4(d.x, d.x, d.y, d.y);
+    m[1] = make_uint4(d.y ^ neg, d.y ^ neg, d.z, d.z);
+    m[2] = make_uint4(d.w, d.w, d.w ^ neg, d.w ^ neg);
+  };
+  // the byte address of tile index i from `first` up, by six bits each
+  auto map_build = [&](uint32_t c, int first, auto column) {
+    if (tid < 128) {
+      const int at = first + (tid < 64 ? 0 : 6), x = tid & 63;
+      uint32_t m = tid < 64 ? c : 0;
+      for (int k = 0; k < 6 && at + k < T; ++k)
+        if ((x >> k) & 1) m ^= column(at + k);
+      (tid < 64 ? map_lo : map_hi)[x] = (uint16_t)m;
+    }
+  };
+  auto addr = [&](uint32_t i) -> uint32_t { return map_lo[i & 63] ^ map_hi[i >> 6]; };
+  if (tid < kChunks) step_put(0, step_chunk(P.gb));
+  map_build(0, 1, [&](int k) { return adj_first_col(k) * kElem; });
+  uint64_t gbase = tile;
+  for (int k = 0; k < P.bits; ++k) gbase = insert_zero(gbase, P.S[k]);
+  __syncthreads();
+  // amplitudes 2e and 2e + 1 of the tile are neighbours (qubit 0 is in every tile)
+  auto pair_at = [&](uint32_t e) { return (gbase | dep_lo[e & 63] | dep_hi[e >> 6]) >> 1; };
+  const uint32_t npairs = 1u << (P.bits - 1);
+  constexpr int kLoads = 4;   // 16-byte loads in flight per thread (of each vector)
+  for (uint32_t e0 = tid; e0 < NT / 2; e0 += kThreads * kLoads) {
+    float4 a[kLoads], l[kLoads];
+#pragma unroll
+    for (int k = 0; k < kLoads; ++k) {
+      const uint32_t e = e0 + kThreads * k;
+      a[k] = l[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (FWD && P.from_zero) {
+        if (e == 0 && gbase == 0) a[k].x = 1.f;
+      } else if (e < npairs) {
+        const uint64_t g = pair_at(e);
+        a[k] = psi[g];
+        if (!FWD) l[k] = lam[g];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kLoads; ++k) {
+      const uint32_t e = e0 + kThreads * k;
+      if (e >= NT / 2) break;
+      const uint32_t A = addr(e);
+      if constexpr (FWD) {
+        el(A) = make_float2(a[k].x, a[k].y);
+        el(A ^ kElem) = make_float2(a[k].z, a[k].w);
+      } else {
+        el(A) = make_float4(a[k].x, l[k].x, a[k].y, l[k].y);
+        el(A ^ kElem) = make_float4(a[k].z, l[k].z, a[k].w, l[k].w);
+      }
+    }
+  }
+  __syncthreads();
+  for (int s = P.gb; s < P.ge; ++s) {
+    const int cur = (s - P.gb) & 1;
+    uint4 pre = make_uint4(0, 0, 0, 0);
+    if (tid < kChunks && s + 1 < P.ge) pre = step_chunk(s + 1);
+    const AdjStep& G = *reinterpret_cast<const AdjStep*>(next[cur]);
+    uint32_t c = G.c;
+    for (int k = 0; k < G.nout; ++k)
+      if ((gbase >> (G.out[k] >> 16)) & 1) c ^= G.out[k] & 0xffffu;
+    double sum[9];
+    bool summed = false;
+    if (G.kind == AG_BLOCK) {
+      const float4* U = reinterpret_cast<const float4*>(next[cur] + 8);
+      uint32_t A0 = c;
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if ((tid >> j) & 1) A0 ^= G.col[j];
+      uint32_t off[1 << kRegs];
+      off[0] = 0;
+#pragma unroll
+      for (int r = 1; r < (1 << kRegs); ++r) off[r] = off[r & (r - 1)] ^ G.v[31 - __clz(r & -r)];
+      const bool sums = !FWD && (G.slot[0] >= 0 || G.slot[1] >= 0 || G.slot[2] >= 0);
+      if (sums) {
+#pragma unroll
+        for (int k = 0; k < 9; ++k) sum[k] = 0.0;
+      }
+      for (uint32_t g = tid; g < (NT >> kRegs); g += kThreads) {
+        const uint32_t A = g & 256u ? A0 ^ G.col[8] : A0;
+        if constexpr (FWD) {
+          float2 w[16];
+#pragma unroll
+          for (int r = 0; r < 16; ++r) w[r] = el(A ^ off[r]);
+          if (G.gates & 1) adj_gate<0>(w, U);
+          if (G.gates & 2) adj_gate<1>(w, U + 2);
+          if (G.gates & 4) adj_gate<2>(w, U + 4);
+          if (G.gates & 8) adj_gate<3>(w, U + 6);
+#pragma unroll
+          for (int r = 0; r < 16; ++r) el(A ^ off[r]) = w[r];
+        } else {
+          float2 re[8], im[8];
+#pragma unroll
+          for (int r = 0; r < 8; ++r) {
+            const float4 p = el(A ^ off[r]);
+            re[r] = make_float2(p.x, p.y);
+            im[r] = make_float2(p.z, p.w);
+          }
+          if (sums) {
+            double2 a[8], l[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+              a[r] = make_double2(re[r].x, im[r].x);
+              l[r] = make_double2(re[r].y, im[r].y);
+            }
+            if (G.slot[0] >= 0) adj_sums<0>(a, l, sum);
+            if (G.slot[1] >= 0) adj_sums<1>(a, l, sum + 3);
+            if (G.slot[2] >= 0) adj_sums<2>(a, l, sum + 6);
+          }
+          if (G.gates & 1) adj_gate<0>(re, im, U);
+          if (G.gates & 2) adj_gate<1>(re, im, U + 6);
+          if (G.gates & 4) adj_gate<2>(re, im, U + 12);
+#pragma unroll
+          for (int r = 0; r < 8; ++r) el(A ^ off[r]) = make_float4(re[r].x, re[r].y, im[r].x, im[r].y);
+        }
+      }
+      if (sums) {
+        const int k = warp_totals<9>(sum, lane);
+        if (k >= 0 && !(lane & 1)) red[cur][tid >> 5][k] = sum[0];
+        summed = true;
+      }
+    } else {
+      // addresses of the tile's indices (of its pairs for a store)
+      map_build(c, G.kind == AG_STORE ? 1 : 0, [&](int k) { return (uint32_t)G.col[k]; });
+      __syncthreads();
+      auto gidx = [&](uint32_t i) { return 2 * pair_at(i >> 1) | (i & 1); };
+      // psi (and lambda) of an element
+      auto get = [&](uint32_t x, float2 (&w)[2]) {
+        if constexpr (FWD) {
+          w[0] = el(x);
+        } else {
+          const float4 p = el(x);
+          w[0] = make_float2(p.x, p.z);
+          w[1] = make_float2(p.y, p.w);
+        }
+      };
+      auto put = [&](uint32_t x, const float2 (&w)[2]) {
+        if constexpr (FWD) el(x) = w[0];
+        else el(x) = make_float4(w[0].x, w[1].x, w[0].y, w[1].y);
+      };
+      constexpr int NV = FWD ? 1 : 2;
+      if (G.kind == AG_STORE) {
+        for (uint32_t e = tid; e < npairs; e += kThreads) {
+          const uint32_t x = addr(e);
+          float2 p[2], q[2];
+          get(x, p);
+          get(x ^ G.col[0], q);
+          const uint64_t g = pair_at(e);
+          psi[g] = make_float4(p[0].x, p[0].y, q[0].x, q[0].y);
+          if (!FWD) lam[g] = make_float4(p[1].x, p[1].y, q[1].x, q[1].y);
+        }
+      } else if (G.kind == AG_MCX) {
+        const int p = G.p0;
+        for (uint32_t k = tid; k < NT / 2; k += kThreads) {
+          const uint32_t i = (uint32_t)insert_zero(k, p);
+          if ((gidx(i) & G.cmask) != G.cmask) continue;
+          const uint32_t x0 = addr(i), x1 = x0 ^ G.col[p];
+          const Elem t = el(x0);
+          el(x0) = el(x1);
+          el(x1) = t;
+        }
+      } else if (G.kind == AG_PHASE) {
+        const float2 ph = FWD ? conjf2(G.ph) : G.ph;
+        for (uint32_t i = tid; i < NT; i += kThreads) {
+          if ((gidx(i) & G.cmask) != G.cmask) continue;
+          float2 w[2];
+          const uint32_t x = addr(i);
+          get(x, w);
+#pragma unroll
+          for (int k = 0; k < NV; ++k) w[k] = G.neg ? make_float2(-w[k].x, -w[k].y) : cmul_comp(w[k], ph);
+          put(x, w);
+        }
+      } else {  // AG_U2
+        Mat4 U = u2[G.mat];
+        if (FWD) {
+          const Mat4 D = U;
+#pragma unroll
+          for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) U.g[4 * r + k] = conjf2(D.g[4 * k + r]);
+        }
+        const int lo2 = min(G.p0, G.p1), hi2 = max(G.p0, G.p1);
+        for (uint32_t k = tid; k < NT / 4; k += kThreads) {
+          const uint32_t x0 = addr((uint32_t)insert_zero(insert_zero(k, lo2), hi2));
+          const uint32_t x[4] = {x0, x0 ^ G.col[G.p0], x0 ^ G.col[G.p1], x0 ^ G.col[G.p0] ^ G.col[G.p1]};
+          float2 w[4][2], o[4][2];
+#pragma unroll
+          for (int r = 0; r < 4; ++r) get(x[r], w[r]);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+#pragma unroll
+            for (int m = 0; m < NV; ++m) o[r][m] = cfma4(U.g + 4 * r, w[0][m], w[1][m], w[2][m], w[3][m]);
+            put(x[r], o[r]);
+          }
+        }
+      }
+    }
+    if (tid < kChunks && s + 1 < P.ge) step_put(cur ^ 1, pre);
+    __syncthreads();
+    if (!FWD && summed && tid < 9 && G.slot[tid / 3] >= 0) {
+      double t = 0.0;
+#pragma unroll
+      for (int w = 0; w < kThreads / 32; ++w) t += red[cur][w][tid];
+      partial[((uint64_t)b * P.nslots + G.slot[tid / 3] + tid % 3) * ntiles + tile] = t;
+    }
+    __syncwarp();   // the step is read above and its buffer refilled by this warp
+  }
+}
+
+// A gate of a run: RX, RY or RZ by its angle, or a constant matrix.
+struct AdjOp { int32_t kind, param, mat, pad; double angle; };
+// A run: its place in the matrix table, its gates in the order they are applied
+// (reverse: undone), the first of its gates' weights.
+struct AdjRun { int32_t row, op0, op1, ref, reverse; };
+
+struct C2 { double re[4], im[4]; };
+__device__ __forceinline__ C2 c2_mul(const C2& a, const C2& b) {
+  C2 c;
+#pragma unroll
+  for (int x = 0; x < 2; ++x)
+#pragma unroll
+    for (int y = 0; y < 2; ++y) {
+      const int p = 2 * x, q = p + 1;
+      c.re[p + y] = a.re[p] * b.re[y] - a.im[p] * b.im[y] + a.re[q] * b.re[2 + y] - a.im[q] * b.im[2 + y];
+      c.im[p + y] = a.re[p] * b.im[y] + a.im[p] * b.re[y] + a.re[q] * b.im[2 + y] + a.im[q] * b.re[2 + y];
+    }
+  return c;
+}
+__device__ __forceinline__ C2 c2_dagger(const C2& a) {
+  return {{a.re[0], a.re[2], a.re[1], a.re[3]}, {-a.im[0], -a.im[2], -a.im[1], -a.im[3]}};
+}
+
+// One thread per (run, vector): the run's matrix (FP64 products, rounded once)
+// and, in the reverse sweep, the axis of each parameter gate as the run's last
+// state sees it.
+__global__ void k_adj_prepare(const AdjRun* __restrict__ runs, int nruns, const AdjOp* __restrict__ ops,
+                              const double* __restrict__ consts, const double* __restrict__ params, int nparams, int nb,
+                              Mat2* __restrict__ mats, double* __restrict__ weights) {
+  const uint64_t id = gtid();
+  if (id >= (uint64_t)nruns * nb) return;
+  const int b = (int)(id % nb);
+  const AdjRun R = runs[id / nb];
+  C2 V{{1, 0, 0, 1}, {0, 0, 0, 0}};   // the gates so far
+  int ref = R.ref;
+  for (int o = R.op0; o < R.op1; ++o) {
+    const AdjOp O = ops[o];
+    C2 U{{0, 0, 0, 0}, {0, 0, 0, 0}};
+    if (O.mat >= 0) {
+      for (int k = 0; k < 4; ++k) { U.re[k] = consts[8 * O.mat + 2 * k]; U.im[k] = consts[8 * O.mat + 2 * k + 1]; }
+    } else {
+      double sn, cs;
+      sincos(0.5 * (O.param >= 0 ? params[(uint64_t)b * nparams + O.param] : O.angle), &sn, &cs);
+      U.re[0] = U.re[3] = cs;
+      if (O.kind == 1) U.im[1] = U.im[2] = -sn;
+      else if (O.kind == 2) { U.re[1] = -sn; U.re[2] = sn; }
+      else { U.im[0] = -sn; U.im[3] = sn; }
+    }
+    if (R.reverse && O.param >= 0) {
+      C2 G{{0, 0, 0, 0}, {0, 0, 0, 0}};
+      if (O.kind == 1) G.re[1] = G.re[2] = 1;
+      else if (O.kind == 2) { G.im[1] = -1; G.im[2] = 1; }
+      else { G.re[0] = 1; G.re[3] = -1; }
+      const C2 A = c2_mul(c2_mul(V, G), c2_dagger(V));   // n . sigma
+      double* w = weights + ((uint64_t)ref * nb + b) * 3;
+      w[0] = A.re[2];
+      w[1] = A.im[2];
+      w[2] = A.re[0];
+      ++ref;
+    }
+    V = R.reverse ? c2_mul(V, U) : c2_mul(U, V);
+  }
+  if (R.reverse) V = c2_dagger(V);
+  Mat2 D;
+  for (int k = 0; k < 4; ++k) D.g[k] = make_float2((float)V.re[k], (float)V.im[k]);
+  mats[(uint64_t)R.row * nb + b] = D;
+}
+
+// A parameter gate: the first of its run's sums, and which weights it has.
+struct AdjRef { int32_t slot, w; };
+
+// grads[b][p] = sum over the gates with parameter p of its axis . (sums over
+// the tiles), one warp per (p, b), in a fixed order.
+__global__ void k_adj_grads(const double* __restrict__ partial, int nslots, uint64_t ntiles,
+                            const int32_t* __restrict__ first, const AdjRef* __restrict__ refs,
+                            const double* __restrict__ weights, int nb, double* __restrict__ grads, int nparams) {
+  const int p = (int)(gtid() >> 5), lane = threadIdx.x & 31, b = blockIdx.y;
+  if (p >= nparams) return;
+  double total = 0.0;
+  for (int k = first[p]; k < first[p + 1]; ++k) {
+    const AdjRef R = refs[k];
+    const double* s = partial + ((uint64_t)b * nslots + R.slot) * ntiles;
+    double x = 0.0, y = 0.0, z = 0.0;
+    for (uint64_t t = lane; t < ntiles; t += 32) {
+      x += s[t];
+      y += s[ntiles + t];
+      z += s[2 * ntiles + t];
+    }
+    const double* w = weights + ((uint64_t)R.w * nb + b) * 3;
+    total += w[0] * warp_sum(x) + w[1] * warp_sum(y) + w[2] * warp_sum(z);
+  }
+  if (lane == 0) grads[(uint64_t)b * nparams + p] = total;
 }
 
 SortedQ sortedq(std::vector<int> q) {
@@ -404,9 +688,6 @@ void mat_1q(const qs_op& o, double theta, cd* m) {
   }
 }
 
-// Reverse-sweep tile width: two staged vectors of 2^12 complex64 = 64 KiB.
-constexpr int kAdjTileBits = 12;
-
 bool adj_passes_enabled() {
   static const bool on = [] {
     const char* e = std::getenv("QSIM_ADJ_PASSES");
@@ -418,6 +699,262 @@ bool adj_passes_enabled() {
 bool is_1q_kind(int k) {
   return k == QS_OP_RX || k == QS_OP_RY || k == QS_OP_RZ || k == QS_OP_U1 || k == QS_OP_DIAG1 || k == QS_OP_Y;
 }
+
+// The passes of a sweep over `order` (op indices): tile qubits by list
+// scheduling, steps by collecting 1Q gates per qubit until a gate needs them done.
+struct AdjPlan {
+  int n, T, L;
+  const qs_op* ops;
+  std::vector<AdjStep> steps;      // each with four rows of the matrix table
+  std::vector<AdjRun> runs;
+  std::vector<AdjOp> run_ops;
+  std::vector<double> consts;      // constant 2x2 matrices
+  std::vector<Mat4> u2s;           // U^dag (the forward kernel transposes it back)
+  std::vector<AdjRef> refs;
+  std::vector<int32_t> ref_param;
+  int nslots = 0;
+
+  // state of the pass that is being cut into steps
+  int pos[64];
+  uint32_t col[kAdjTileBits], cst;
+  std::vector<std::pair<int, uint32_t>> out;
+  std::vector<int> pending[kAdjTileBits];
+  bool reverse;
+  int regs;                        // positions of a block
+  uint32_t elem;                   // bytes of a tile element
+
+  AdjStep step(int kind) {
+    AdjStep G;
+    std::memset(&G, 0, sizeof(G));
+    G.kind = kind;
+    G.c = (uint16_t)(cst * elem);
+    G.slot[0] = G.slot[1] = G.slot[2] = -1;
+    for (const auto& o : out)
+      if (o.second) G.out[G.nout++] = (uint32_t)o.first << 16 | o.second * elem;
+    for (int k = 0; k < T; ++k) G.col[k] = (uint16_t)(col[k] * elem);
+    return G;
+  }
+
+  // The pending gates of up to `regs` positions as one block.
+  void block(const int* which, int count) {
+    int bits[4];
+    bool used[kAdjTileBits] = {};
+    for (int j = 0; j < count; ++j) { bits[j] = which[j]; used[which[j]] = true; }
+    for (int j = count, k = T - 1; j < regs; --k)
+      if (!used[k]) { bits[j++] = k; used[k] = true; }
+    AdjStep G = step(AG_BLOCK);
+    for (int j = 0; j < regs; ++j) G.v[j] = (uint16_t)(col[bits[j]] * elem);
+    // thread bits: first those whose columns spread the lanes of one access
+    // over the banks (8 elements of 16 bytes or 16 of 8)
+    const uint32_t low = reverse ? 7u : 15u;
+    std::vector<uint32_t> basis, lead, rest;
+    for (int k = 0; k < T; ++k) {
+      if (used[k]) continue;
+      uint32_t x = col[k] & low;
+      for (uint32_t e : basis) x = std::min(x, x ^ e);
+      if (x) { basis.push_back(x); lead.push_back(col[k]); } else rest.push_back(col[k]);
+    }
+    std::memset(G.col, 0, sizeof(G.col));
+    int j = 0;
+    for (uint32_t x : lead) G.col[j++] = (uint16_t)(x * elem);
+    for (uint32_t x : rest) G.col[j++] = (uint16_t)(x * elem);
+    steps.push_back(G);
+    AdjStep& S = steps.back();
+    for (int q = 0; q < count; ++q) {
+      std::vector<int>& run = pending[which[q]];
+      S.gates |= 1u << q;
+      AdjRun R{(int32_t)(4 * (steps.size() - 1)) + q, (int32_t)run_ops.size(), 0, (int32_t)refs.size(), reverse};
+      for (int o : run) {
+        run_ops.push_back(run_op(ops[o]));
+        if (!reverse || ops[o].param < 0) continue;
+        refs.push_back(AdjRef{nslots, (int32_t)refs.size()});
+        ref_param.push_back(ops[o].param);
+      }
+      if ((int32_t)refs.size() > R.ref) {
+        S.slot[q] = nslots;
+        nslots += 3;
+      }
+      R.op1 = (int32_t)run_ops.size();
+      runs.push_back(R);
+      run.clear();
+    }
+  }
+
+  AdjOp run_op(const qs_op& o) {
+    AdjOp O{o.kind == QS_OP_RX ? 1 : o.kind == QS_OP_RY ? 2 : 3, o.param, -1, 0, o.m[0]};
+    if (o.kind == QS_OP_RX || o.kind == QS_OP_RY || o.kind == QS_OP_RZ) return O;
+    cd m[4];
+    mat_1q(o, 0.0, m);
+    O.param = -1;
+    O.mat = (int32_t)(consts.size() / 8);
+    for (const cd& x : m) { consts.push_back(x.real()); consts.push_back(x.imag()); }
+    return O;
+  }
+
+  // Runs the pending gates of the tile positions in `need`; free places of a
+  // block go to the positions that a later op of the pass needs first.
+  void flush(uint32_t need, const std::vector<int>& cur, size_t at) {
+    int which[4], count = 0;
+    uint32_t taken = 0;
+    auto take = [&](int p) {
+      which[count++] = p;
+      taken |= 1u << p;
+      if (count == regs) { block(which, regs); count = 0; }
+    };
+    bool any = false;
+    for (int p = 0; p < T; ++p)
+      if (((need >> p) & 1) && !pending[p].empty()) { take(p); any = true; }
+    if (!any || count == 0) return;
+    uint32_t open = 0;   // positions that get more gates before they are needed
+    for (size_t k = at; k < cur.size() && count > 0; ++k) {
+      const qs_op& o = ops[cur[k]];
+      for (int q = 0; q < o.nq && count > 0; ++q) {
+        const int p = pos[o.q[q]];
+        if (p < 0) continue;
+        if (is_1q_kind(o.kind)) open |= 1u << p;
+        else if (!((open | taken) >> p & 1) && !pending[p].empty()) take(p);
+      }
+    }
+    for (int p = 0; p < T && count > 0; ++p)
+      if (!((open | taken) >> p & 1) && !pending[p].empty()) take(p);
+    if (count) block(which, count);
+  }
+
+  void pass(uint64_t S, const std::vector<int>& cur, std::vector<PassArg>& passes) {
+    PassArg P;
+    std::memset(&P, 0, sizeof(P));
+    P.T = T;
+    P.bits = std::min(n, T);
+    std::fill(pos, pos + 64, -1);
+    int k = 0;
+    for (int q = 0; q < n; ++q)
+      if ((S >> q) & 1) { P.S[k] = q; pos[q] = k++; }
+    for (int j = 0; j < T; ++j) col[j] = adj_first_col(j);
+    cst = 0;
+    out.clear();
+    P.gb = (int)steps.size();
+    for (size_t at = 0; at < cur.size(); ++at) {
+      const int i = cur[at];
+      const qs_op& o = ops[i];
+      if (is_1q_kind(o.kind)) {
+        pending[pos[o.q[0]]].push_back(i);
+        continue;
+      }
+      uint32_t need = 0;
+      for (int q = 0; q < o.nq; ++q)
+        if (pos[o.q[q]] >= 0) need |= 1u << pos[o.q[q]];
+      flush(need, cur, at + 1);
+      if (o.kind == QS_OP_MCX && o.nq <= 2) {
+        const int t = pos[o.q[o.nq - 1]], c = o.nq == 2 ? pos[o.q[0]] : -1;
+        if (o.nq == 1) { cst ^= col[t]; continue; }
+        if (c >= 0) { col[c] ^= col[t]; continue; }
+        size_t e = 0;
+        while (e < out.size() && out[e].first != o.q[0]) ++e;
+        if (e == out.size() && e < (size_t)kAdjOut) out.push_back({o.q[0], 0u});
+        if (e < out.size()) { out[e].second ^= col[t]; continue; }
+        // more controls outside the tile than a step holds: a sweep
+      }
+      AdjStep G = step(o.kind == QS_OP_MCX ? AG_MCX : o.kind == QS_OP_MCPHASE ? AG_PHASE : AG_U2);
+      if (o.kind == QS_OP_MCX) {
+        G.p0 = (uint8_t)pos[o.q[o.nq - 1]];
+        for (int q = 0; q + 1 < o.nq; ++q) G.cmask |= 1ull << o.q[q];
+      } else if (o.kind == QS_OP_MCPHASE) {
+        for (int q = 0; q < o.nq; ++q) G.cmask |= 1ull << o.q[q];
+        G.neg = (o.m[0] == -1.0 && o.m[1] == 0.0) ? 1 : 0;
+        G.ph = make_float2((float)o.m[0], (float)-o.m[1]);
+      } else {
+        G.p0 = (uint8_t)pos[o.q[0]];
+        G.p1 = (uint8_t)pos[o.q[1]];
+        G.mat = (int)u2s.size();
+        Mat4 U;
+        for (int r = 0; r < 4; ++r)
+          for (int q = 0; q < 4; ++q)
+            U.g[4 * r + q] = make_float2((float)o.m[2 * (4 * q + r)], (float)-o.m[2 * (4 * q + r) + 1]);
+        u2s.push_back(U);
+      }
+      steps.push_back(G);
+    }
+    int which[4], count = 0;
+    for (int p = 0; p < T; ++p) {
+      if (pending[p].empty()) continue;
+      which[count++] = p;
+      if (count == regs) { block(which, regs); count = 0; }
+    }
+    if (count) block(which, count);
+    steps.push_back(step(AG_STORE));
+    P.ge = (int)steps.size();
+    passes.push_back(P);
+  }
+
+  // List scheduling: an op is ready when it is the next op of the order on
+  // every qubit it touches (ops on disjoint qubits commute, and so do their
+  // contributions to the gradient); a pass keeps taking ready ops whose targets
+  // are in its tile, and adds the targets of the earliest ready op to the tile
+  // while room is left.
+  void sweep(const std::vector<int>& order, bool rev, std::vector<PassArg>& passes) {
+    reverse = rev;
+    regs = rev ? 3 : 4;
+    elem = rev ? sizeof(float4) : sizeof(float2);
+    const int m = (int)order.size(), bits = std::min(n, T);
+    std::vector<uint64_t> touch(m), targ(m);
+    std::vector<std::vector<int>> per_q(n);   // positions in `order` touching each qubit
+    for (int k = 0; k < m; ++k) {
+      const qs_op& o = ops[order[k]];
+      for (int q = 0; q < o.nq; ++q) {
+        touch[k] |= 1ull << o.q[q];
+        per_q[o.q[q]].push_back(k);
+      }
+      if (is_1q_kind(o.kind)) targ[k] = 1ull << o.q[0];
+      else if (o.kind == QS_OP_MCX) targ[k] = 1ull << o.q[o.nq - 1];
+      else if (o.kind == QS_OP_U2) targ[k] = 1ull << o.q[0] | 1ull << o.q[1];
+    }
+    std::vector<size_t> head(n, 0);   // next unscheduled position per qubit
+    std::vector<char> done(m, 0);
+    auto ready = [&](int k) {
+      for (uint64_t t = touch[k]; t; t &= t - 1) {
+        const int q = __builtin_ctzll(t);
+        if (per_q[q][head[q]] != k) return false;
+      }
+      return true;
+    };
+    const uint64_t lows = (1ull << (bits == n ? n : L)) - 1;
+    uint64_t S = lows;
+    std::vector<int> cur;
+    auto close = [&]() {
+      for (int q = 0; __builtin_popcountll(S) < bits && q < n; ++q) S |= 1ull << q;  // fill the tile
+      // back in the order of the sweep (it respects every dependency): taken as
+      // the tile grew, a layer's gates would be scattered over many blocks
+      std::sort(cur.begin(), cur.end());
+      for (int& k : cur) k = order[k];
+      if (!cur.empty()) pass(S, cur, passes);
+      cur.clear();
+      S = lows;
+    };
+    int remaining = m, first = 0;
+    while (remaining > 0) {
+      bool progress = true;
+      while (progress) {
+        progress = false;
+        for (int k = first; k < m; ++k) {
+          if (done[k] || (targ[k] & ~S) || !ready(k)) continue;
+          done[k] = 1;
+          --remaining;
+          for (uint64_t t = touch[k]; t; t &= t - 1) ++head[__builtin_ctzll(t)];
+          cur.push_back(k);
+          progress = true;
+        }
+        while (first < m && done[first]) ++first;
+      }
+      if (remaining == 0) break;
+      // widen the tile with the earliest ready op's targets, or close the pass
+      int pick = first;
+      while (done[pick] || !ready(pick)) ++pick;
+      if (__builtin_popcountll(S | targ[pick]) <= bits) S |= targ[pick];
+      else close();
+    }
+    close();
+  }
+};
 
 }  // namespace
 
@@ -447,203 +984,106 @@ extern "C" int qs_adjoint_gradient(qs_handle_t h, int n, const qs_op* ops, int n
                    "only RX/RY/RZ ops may carry a parameter");
     QS_CHECK_ARG(is_1q_kind(o.kind) || o.kind == QS_OP_MCX || o.kind == QS_OP_MCPHASE || o.kind == QS_OP_U2,
                  "op kind not supported by the adjoint sweep");
+    QS_CHECK_ARG(o.nq >= 1 && o.nq <= 8, "bad qubit count");
+    for (int q = 0; q < o.nq; ++q) qs_check_qubit(o.q[q], n, "op");
   }
-  // The pass sweeps keep one FP64 partial per (vector, parameter gate, tile);
-  // past 1 GiB of partials the per-gate sweep (partials per block) is used.
-  size_t n_param_gates = 0;
-  for (int i = 0; i < nops; ++i) n_param_gates += (ops[i].param >= 0 && is_1q_kind(ops[i].kind)) ? 1 : 0;
-  const int T = std::min(n, kAdjTileBits);
-  const uint64_t ntiles = 1ull << (n - T);
-  const bool use_passes = adj_passes_enabled() &&
-      (double)nb * (double)std::max<size_t>(n_param_gates, 1) * (double)ntiles * sizeof(double) <=
-          (double)(1ull << 30);
+  // Tiles of at least the register bits of a block; the low qubits in every
+  // tile make its runs of global memory whole 128-byte lines.
+  const int T = std::max(4, std::min(n, kAdjTileBits));
+  const uint64_t ntiles = 1ull << std::max(0, n - T);
+  AdjPlan plan{n, T, std::min(n, kAdjLowQubits), ops};
+  std::vector<PassArg> fpasses, rpasses;
+  bool use_passes = adj_passes_enabled();
+  if (use_passes) {
+    std::vector<int> order(nops);
+    for (int i = 0; i < nops; ++i) order[i] = i;
+    plan.sweep(order, false, fpasses);
+    std::reverse(order.begin(), order.end());
+    plan.sweep(order, true, rpasses);
+    fpasses[0].from_zero = 1;
+    for (auto& P : rpasses) P.nslots = plan.nslots;
+    // one FP64 partial per (vector, sum, tile); past 1.5 GiB of them the
+    // per-gate sweep (partials per block) is used
+    use_passes = (double)nb * std::max(plan.nslots, 1) * (double)ntiles * sizeof(double) <= 1.5 * (double)(1ull << 30);
+  }
 
-  // device buffer: grads [nb][nparams] | energies [nb] | partial [nb][256] | U^dag tables
+  // device buffer: grads [nb][nparams] | energies [nb] | partial [nb][256] | U^dag table of the per-gate sweep
   const size_t ng = (size_t)nb * std::max(nparams, 1);
   const Slice sl = slice(N / 2);
   const Slice sd = slice(N);
   const int nbx = std::max(sl.nbx, sd.nbx);
-  size_t bytes = sizeof(double) * (ng + nb + (size_t)nb * nbx) + sizeof(Mat2) * (size_t)nb * nops + 64;
+  std::vector<Mat2> udag(use_passes ? 0 : (size_t)nb * nops);
+  const size_t bytes = sizeof(double) * (ng + nb + (size_t)nb * nbx) + sizeof(Mat2) * udag.size() + 64;
   QS_CUDA(cudaMallocAsync(&dbuf, bytes, h->stream));
   double* d_grads = (double*)dbuf;
   double* d_energy = d_grads + ng;
   double* d_part = d_energy + nb;
   Mat2* d_udag = (Mat2*)(((uintptr_t)(d_part + (size_t)nb * nbx) + 15) & ~uintptr_t(15));
   QS_CUDA(cudaMemsetAsync(d_grads, 0, sizeof(double) * ng, h->stream));
-
-  // per-(op, b) U^dag for the 1Q ops
-  std::vector<Mat2> udag((size_t)nb * nops);
-  for (int i = 0; i < nops; ++i) {
+  for (int i = 0; i < nops && !use_passes; ++i) {
     if (!is_1q_kind(ops[i].kind)) continue;
     for (int b = 0; b < nb; ++b) {
-      const double th = ops[i].param >= 0 ? params[(size_t)b * nparams + ops[i].param] : ops[i].m[0];
       cd m[4];
-      mat_1q(ops[i], th, m);
-      Mat2& U = udag[(size_t)i * nb + b];
-      // conjugate transpose
-      U.g[0] = make_float2((float)m[0].real(), (float)-m[0].imag());
-      U.g[1] = make_float2((float)m[2].real(), (float)-m[2].imag());
-      U.g[2] = make_float2((float)m[1].real(), (float)-m[1].imag());
-      U.g[3] = make_float2((float)m[3].real(), (float)-m[3].imag());
+      mat_1q(ops[i], ops[i].param >= 0 ? params[(size_t)b * nparams + ops[i].param] : ops[i].m[0], m);
+      for (int k = 0; k < 4; ++k) {   // conjugate transpose
+        const cd x = m[2 * (k & 1) + (k >> 1)];
+        udag[(size_t)i * nb + b].g[k] = make_float2((float)x.real(), (float)-x.imag());
+      }
     }
   }
-  QS_CUDA(cudaMemcpyAsync(d_udag, udag.data(), sizeof(Mat2) * udag.size(), cudaMemcpyHostToDevice, h->stream));
+  if (!udag.empty())
+    QS_CUDA(cudaMemcpyAsync(d_udag, udag.data(), sizeof(Mat2) * udag.size(), cudaMemcpyHostToDevice, h->stream));
 
-  // ---- tile passes (forward order and reverse order)
-  std::vector<AdjGate> gates;
-  std::vector<PassArg> fpasses, rpasses;
-  std::vector<int32_t> param_of;
-  std::vector<Mat4> u2s;
-  AdjGate* d_gates = nullptr;
+  AdjStep* d_steps = nullptr;
+  float4* d_mats = nullptr;
   Mat4* d_u2 = nullptr;
-  int32_t* d_param_of = nullptr;
-  double* d_parts = nullptr;
-  size_t pass_smem[2] = {0, 0};
+  AdjRef* d_refs = nullptr;
+  int32_t* d_first = nullptr;
+  double *d_weights = nullptr, *d_parts = nullptr;
+  const size_t pass_smem[2] = {sizeof(float2) << T, sizeof(float4) << T};
   if (use_passes) {
-    const int L = std::min(n, 5);  // low qubits always in the tile (coalesced runs)
-    // Greedy cut of an op sequence into passes: a pass takes ops in order
-    // while their targets fit in T tile qubits.
-    auto build = [&](const std::vector<int>& order, bool reverse, std::vector<PassArg>& out) {
-      std::set<int> S;
-      std::vector<int> cur;
-      auto reset_S = [&]() {
-        S.clear();
-        for (int q = 0; q < (T == n ? n : L); ++q) S.insert(q);
-      };
-      auto close_pass = [&]() {
-        if (cur.empty()) { reset_S(); return; }
-        for (int q = 0; (int)S.size() < T && q < n; ++q) S.insert(q);  // fill the tile to T qubits
-        PassArg P;
-        std::memset(&P, 0, sizeof(P));
-        P.T = T;
-        int k = 0, pos[64];
-        for (int q : S) { P.S[k] = q; pos[q] = k; ++k; }
-        P.gb = (int)gates.size();
-        for (int i : cur) {
-          const qs_op& o = ops[i];
-          AdjGate G;
-          std::memset(&G, 0, sizeof(G));
-          G.slot = -1;
-          if (is_1q_kind(o.kind)) {
-            G.kind = AG_1Q;
-            G.p0 = pos[o.q[0]];
-            G.mat = i;
-            if (reverse && o.param >= 0) {
-              G.gkind = o.kind == QS_OP_RX ? 1 : o.kind == QS_OP_RY ? 2 : 3;
-              G.slot = (int)param_of.size();
-              param_of.push_back(o.param);
-            }
-          } else if (o.kind == QS_OP_MCX) {
-            G.kind = AG_MCX;
-            G.p0 = pos[o.q[o.nq - 1]];
-            for (int c = 0; c + 1 < o.nq; ++c) G.cmask |= 1ull << o.q[c];
-          } else if (o.kind == QS_OP_MCPHASE) {
-            G.kind = AG_PHASE;
-            for (int c = 0; c < o.nq; ++c) G.cmask |= 1ull << o.q[c];
-            G.neg = (o.m[0] == -1.0 && o.m[1] == 0.0) ? 1 : 0;
-            G.ph = make_float2((float)o.m[0], (float)-o.m[1]);
-          } else {
-            G.kind = AG_U2;
-            G.p0 = pos[o.q[0]];
-            G.p1 = pos[o.q[1]];
-            G.mat = (int)u2s.size();
-            Mat4 U;  // U^dag; the forward kernel transposes it back
-            for (int r = 0; r < 4; ++r)
-              for (int c = 0; c < 4; ++c)
-                U.g[4 * r + c] = make_float2((float)o.m[2 * (4 * c + r)], (float)-o.m[2 * (4 * c + r) + 1]);
-            u2s.push_back(U);
-          }
-          gates.push_back(G);
-        }
-        P.ge = (int)gates.size();
-        out.push_back(P);
-        cur.clear();
-        reset_S();
-      };
-      // List scheduling: an op is ready when it is the next op of the order
-      // on every qubit it touches (ops on disjoint qubits commute, and so do
-      // their contributions to the gradient); a pass keeps taking ready ops
-      // whose targets are in its tile, and adds the targets of the earliest
-      // ready op to the tile while room is left.
-      const int m = (int)order.size();
-      std::vector<std::vector<int>> touch(m), targ(m);
-      std::vector<std::vector<int>> per_q(n);  // positions in `order` touching each qubit
-      for (int k = 0; k < m; ++k) {
-        const qs_op& o = ops[order[k]];
-        if (is_1q_kind(o.kind)) targ[k] = {o.q[0]};
-        else if (o.kind == QS_OP_MCX) targ[k] = {o.q[o.nq - 1]};
-        else if (o.kind == QS_OP_U2) targ[k] = {o.q[0], o.q[1]};
-        touch[k].assign(o.q, o.q + o.nq);
-        for (int q : touch[k]) per_q[q].push_back(k);
-      }
-      std::vector<size_t> head(n, 0);  // next unscheduled position per qubit
-      std::vector<char> done(m, 0);
-      auto ready = [&](int k) {
-        for (int q : touch[k])
-          if (per_q[q][head[q]] != k) return false;
-        return true;
-      };
-      auto fits = [&](int k) {
-        for (int q : targ[k])
-          if (!S.count(q)) return false;
-        return true;
-      };
-      int remaining = m, first = 0;
-      reset_S();
-      while (remaining > 0) {
-        bool progress = true;
-        while (progress) {
-          progress = false;
-          for (int k = first; k < m; ++k) {
-            if (done[k] || !ready(k) || !fits(k)) continue;
-            done[k] = 1;
-            --remaining;
-            for (int q : touch[k]) ++head[q];
-            cur.push_back(order[k]);
-            progress = true;
-          }
-          while (first < m && done[first]) ++first;
-        }
-        if (remaining == 0) break;
-        // widen the tile with the earliest ready op's targets, or close the pass
-        int pick = -1;
-        for (int k = first; k < m && pick < 0; ++k)
-          if (!done[k] && ready(k)) pick = k;
-        std::set<int> need = S;
-        need.insert(targ[pick].begin(), targ[pick].end());
-        if ((int)need.size() <= T) {
-          S = need;
-        } else {
-          close_pass();
-        }
-      }
-      close_pass();
+    // the gates of each parameter, in the order of the sweep
+    std::vector<int32_t> pfirst(nparams + 1, 0);
+    for (int32_t p : plan.ref_param) ++pfirst[p + 1];
+    for (int p = 0; p < nparams; ++p) pfirst[p + 1] += pfirst[p];
+    std::vector<AdjRef> refs(plan.refs.size());
+    std::vector<int32_t> fill(pfirst);
+    for (size_t k = 0; k < refs.size(); ++k) refs[fill[plan.ref_param[k]]++] = plan.refs[k];
+    std::vector<char> host;
+    size_t off[8];
+    auto put = [&](int k, const void* d, size_t size) {
+      off[k] = host.size();
+      host.resize((host.size() + size + 255) & ~size_t(255));
+      if (size) std::memcpy(host.data() + off[k], d, size);
     };
-    std::vector<int> order(nops);
-    for (int i = 0; i < nops; ++i) order[i] = i;
-    build(order, false, fpasses);
-    std::reverse(order.begin(), order.end());
-    build(order, true, rpasses);
-    if (!fpasses.empty()) fpasses[0].from_zero = 1;
-    const int nslots = (int)param_of.size();
-    for (auto& P : rpasses) P.nslots = nslots;
-    // device: gates | U2 matrices | slot -> parameter | partials
-    const size_t gbytes = gates.size() * sizeof(AdjGate), ubytes = u2s.size() * sizeof(Mat4);
-    const size_t pbytes = sizeof(int32_t) * std::max(nslots, 1);
-    const size_t parts = (size_t)nb * std::max(nslots, 1) * ntiles;
-    auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
-    QS_CUDA(cudaMallocAsync(&pbuf, al(gbytes) + al(ubytes) + al(pbytes) + sizeof(double) * parts, h->stream));
+    put(0, plan.steps.data(), plan.steps.size() * sizeof(AdjStep));
+    put(1, plan.runs.data(), plan.runs.size() * sizeof(AdjRun));
+    put(2, plan.u2s.data(), plan.u2s.size() * sizeof(Mat4));
+    put(3, refs.data(), refs.size() * sizeof(AdjRef));
+    put(4, pfirst.data(), pfirst.size() * sizeof(int32_t));
+    put(5, plan.run_ops.data(), plan.run_ops.size() * sizeof(AdjOp));
+    put(6, plan.consts.data(), plan.consts.size() * sizeof(double));
+    put(7, params, sizeof(double) * (size_t)nb * nparams);
+    const size_t parts = (size_t)nb * std::max(plan.nslots, 1) * ntiles, nmats = plan.steps.size() * 4 * nb;
+    QS_CUDA(cudaMallocAsync(&pbuf, host.size() + sizeof(Mat2) * nmats +
+                            sizeof(double) * (parts + 3 * (size_t)nb * refs.size()), h->stream));
     char* pc = static_cast<char*>(pbuf);
-    d_gates = reinterpret_cast<AdjGate*>(pc);
-    d_u2 = reinterpret_cast<Mat4*>(pc + al(gbytes));
-    d_param_of = reinterpret_cast<int32_t*>(pc + al(gbytes) + al(ubytes));
-    d_parts = reinterpret_cast<double*>(pc + al(gbytes) + al(ubytes) + al(pbytes));
-    if (gbytes) QS_CUDA(cudaMemcpyAsync(d_gates, gates.data(), gbytes, cudaMemcpyHostToDevice, h->stream));
-    if (ubytes) QS_CUDA(cudaMemcpyAsync(d_u2, u2s.data(), ubytes, cudaMemcpyHostToDevice, h->stream));
-    if (nslots)
-      QS_CUDA(cudaMemcpyAsync(d_param_of, param_of.data(), pbytes, cudaMemcpyHostToDevice, h->stream));
-    pass_smem[0] = sizeof(float2) * ((size_t)1 << T) + 2 * 128 * sizeof(uint64_t);  // forward
-    pass_smem[1] = sizeof(float2) * 2 * ((size_t)1 << T) + 2 * 128 * sizeof(uint64_t);
+    d_steps = reinterpret_cast<AdjStep*>(pc + off[0]);
+    d_mats = reinterpret_cast<float4*>(pc + host.size());
+    d_u2 = reinterpret_cast<Mat4*>(pc + off[2]);
+    d_refs = reinterpret_cast<AdjRef*>(pc + off[3]);
+    d_first = reinterpret_cast<int32_t*>(pc + off[4]);
+    d_parts = reinterpret_cast<double*>(pc + host.size() + sizeof(Mat2) * nmats);
+    d_weights = d_parts + parts;
+    QS_CUDA(cudaMemcpyAsync(pc, host.data(), host.size(), cudaMemcpyHostToDevice, h->stream));
+    const int nruns = (int)plan.runs.size();
+    if (nruns) {
+      k_adj_prepare<<<(unsigned)(((uint64_t)nruns * nb + 127) / 128), 128, 0, h->stream>>>(
+          reinterpret_cast<AdjRun*>(pc + off[1]), nruns, reinterpret_cast<AdjOp*>(pc + off[5]),
+          reinterpret_cast<double*>(pc + off[6]), reinterpret_cast<double*>(pc + off[7]), nparams, nb, (Mat2*)d_mats,
+          d_weights);
+      qs_after_launch(h, "k_adj_prepare");
+    }
     QS_CUDA(cudaFuncSetAttribute(k_adj_pass<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_smem[0]));
     QS_CUDA(cudaFuncSetAttribute(k_adj_pass<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_smem[1]));
   }
@@ -652,7 +1092,7 @@ extern "C" int qs_adjoint_gradient(qs_handle_t h, int n, const qs_op* ops, int n
   if (use_passes) {
     for (const PassArg& P : fpasses) {
       k_adj_pass<true><<<dim3((unsigned)ntiles, nb), kThreads, pass_smem[0], h->stream>>>(
-          (float2*)work, vstride, P, d_gates, d_udag, nb, d_u2, nullptr);
+          (float2*)work, vstride, P, d_steps, d_mats, nb, d_u2, nullptr);
       qs_after_launch(h, "k_adj_pass");
     }
   } else {
@@ -689,13 +1129,13 @@ extern "C" int qs_adjoint_gradient(qs_handle_t h, int n, const qs_op* ops, int n
   if (use_passes) {
     for (const PassArg& P : rpasses) {
       k_adj_pass<false><<<dim3((unsigned)ntiles, nb), kThreads, pass_smem[1], h->stream>>>(
-          (float2*)work, vstride, P, d_gates, d_udag, nb, d_u2, d_parts);
+          (float2*)work, vstride, P, d_steps, d_mats, nb, d_u2, d_parts);
       qs_after_launch(h, "k_adj_pass");
     }
-    if (!param_of.empty()) {
-      k_adj_slots<<<nb, kThreads, 0, h->stream>>>(d_parts, (int)param_of.size(), ntiles, d_param_of, d_grads,
-                                                  nparams);
-      qs_after_launch(h, "k_adj_slots");
+    if (nparams > 0) {
+      k_adj_grads<<<dim3((unsigned)((nparams + 3) / 4), nb), 128, 0, h->stream>>>(
+          d_parts, plan.nslots, ntiles, d_first, d_refs, d_weights, nb, d_grads, nparams);
+      qs_after_launch(h, "k_adj_grads");
     }
   } else
   for (int i = nops - 1; i >= 0; --i) {
