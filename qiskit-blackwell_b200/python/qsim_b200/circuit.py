@@ -11,7 +11,9 @@ converts a real QuantumCircuit when qiskit is installed.
 """
 from __future__ import annotations
 
+import cmath
 import math
+import struct
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -236,11 +238,79 @@ def _set_m(rec, mat):
     rec["m"][1: 2 * flat.size: 2] = flat.imag
 
 
+# One record is packed at a time into bytes (OP_DTYPE's layout) and the array
+# made from them at the end: assigning the fields of a structured array costs
+# about 8 us per op, packing 1-2.
+_HEAD = struct.Struct("<12i")       # kind, nq, q[8], param, flags
+_SCALAR = struct.Struct("<d")
+_PHASE = struct.Struct("<2d")
+_DIAG = struct.Struct("<4d")
+_MAT = struct.Struct("<8d")
+_NO_QUBITS = tuple((0,) * k for k in range(9))
+_ZEROS = bytes(256)                 # m when empty
+_ROTATIONS = {"rx": OP_RX, "ry": OP_RY, "rz": OP_RZ}
+_MCX_NAMES = frozenset(("cx", "cnot", "ccx", "toffoli", "mcx", "c3x", "c4x"))
+
+
+def _pack_m(mat) -> bytes:
+    return np.asarray(mat, dtype=np.complex128).tobytes()
+
+
+def _lower_one(ins) -> tuple:
+    """(kind, parameter index, bytes of m) of one gate."""
+    name = ins.name
+    if name == "unitary":
+        return (OP_U1 if len(ins.qubits) == 1 else OP_U2), -1, _pack_m(ins.matrix)
+    if name in NOISE_OPS:
+        return NOISE_OPS[name], -1, _SCALAR.pack(float(ins.params[0]))
+    if name in _MCX_NAMES:
+        return OP_MCX, -1, b""
+    if name == "cz":
+        return OP_MCPHASE, -1, _SCALAR.pack(-1.0)
+    if name in _ROTATIONS and ins.param_index >= 0:
+        return _ROTATIONS[name], ins.param_index, _SCALAR.pack(float(ins.params[0]))
+    if name == "rz":
+        a, b = cmath.exp(-0.5j * float(ins.params[0])), cmath.exp(0.5j * float(ins.params[0]))
+        return OP_DIAG1, -1, _DIAG.pack(a.real, a.imag, b.real, b.imag)
+    if name == "ry":
+        c, s = math.cos(float(ins.params[0]) / 2), math.sin(float(ins.params[0]) / 2)
+        return OP_U1, -1, _MAT.pack(c, 0.0, -s, 0.0, s, 0.0, c, 0.0)
+    if name == "y":
+        return OP_Y, -1, b""
+    if name in G.DIAGONAL_1Q:
+        m = G.mat1(name, ins.params)
+        return OP_DIAG1, -1, _pack_m([m[0, 0], m[1, 1]])
+    if name in G.NATIVE_1Q:
+        return OP_U1, -1, _pack_m(G.mat1(name, ins.params))
+    if name == "cp":
+        return OP_MCPHASE, -1, _PHASE.pack(math.cos(ins.params[0]), math.sin(ins.params[0]))
+    if name in ("swap", "cswap"):
+        return OP_MCSWAP, -1, b""
+    if name == "crz":
+        return OP_MCU1, -1, _pack_m(G.mat1("rz", ins.params))
+    if name == "cu":
+        return OP_MCU1, -1, _pack_m(G.cu_target(ins.params))
+    if name in G.CONTROLLED_1Q:
+        return OP_MCU1, -1, _pack_m(G.mat1(G.CONTROLLED_1Q[name], ins.params))
+    if name in G.CONTROLLED_PHASE:
+        return OP_MCPHASE, -1, _pack_m(complex(G.CONTROLLED_PHASE[name](ins.params)))
+    if name == "rzz":
+        return OP_DIAG2, -1, _pack_m(np.diagonal(G.pauli_rot2("z", "z", float(ins.params[0]))))
+    if name in G.PAULI_ROT_2Q:
+        return OP_U2, -1, _pack_m(G.pauli_rot2(*G.PAULI_ROT_2Q[name], float(ins.params[0])))
+    if name == "iswap":
+        return OP_U2, -1, _pack_m(G.ISWAP)
+    if name == "r":
+        return OP_U1, -1, _pack_m(G.r_gate(float(ins.params[0]), float(ins.params[1])))
+    if name == "mcu":
+        return (OP_MCU1 if int(ins.params[0]) == 1 else OP_MCU2), -1, _pack_m(ins.matrix)
+    raise ValueError(f"Unsupported instruction: {name}")
+
+
 def lower(circuit: Circuit, strip_measure: bool = True) -> np.ndarray:
     """Circuit -> qs_op structured array (measure/reset/barrier dropped when
     strip_measure, else rejected; they are handled by the backend)."""
-    recs = np.zeros(2 * len(circuit.data), dtype=OP_DTYPE)
-    k = 0
+    parts = []
     for ins in circuit.data:
         name, qs = ins.name, ins.qubits
         if name == "barrier":
@@ -249,79 +319,19 @@ def lower(circuit: Circuit, strip_measure: bool = True) -> np.ndarray:
             if strip_measure:
                 continue
             raise ValueError("measure/reset cannot be lowered to a unitary program")
-        r = recs[k]
-        r["param"] = -1
-        r["nq"] = len(qs)
-        r["q"][: len(qs)] = qs
-        if name in ("rx", "ry", "rz") and ins.param_index >= 0:
-            r["kind"] = {"rx": OP_RX, "ry": OP_RY, "rz": OP_RZ}[name]
-            r["m"][0] = float(ins.params[0])
-            r["param"] = ins.param_index
-        elif name == "unitary":
-            r["kind"] = OP_U1 if len(qs) == 1 else OP_U2
-            _set_m(r, ins.matrix)
-        elif name in NOISE_OPS:
-            r["kind"] = NOISE_OPS[name]
-            r["m"][0] = float(ins.params[0])
-        elif name == "y":
-            r["kind"] = OP_Y
-        elif name in G.DIAGONAL_1Q:
-            r["kind"] = OP_DIAG1
-            m = G.mat1(name, ins.params)
-            _set_m(r, [m[0, 0], m[1, 1]])
-        elif name in G.NATIVE_1Q:
-            r["kind"] = OP_U1
-            _set_m(r, G.mat1(name, ins.params))
-        elif name in ("cx", "cnot", "ccx", "toffoli", "mcx", "c3x", "c4x"):
-            r["kind"] = OP_MCX
-        elif name == "cz":
-            r["kind"] = OP_MCPHASE
-            _set_m(r, [-1.0])
-        elif name == "cp":
-            r["kind"] = OP_MCPHASE
-            _set_m(r, [complex(math.cos(ins.params[0]), math.sin(ins.params[0]))])
-        elif name == "swap":
-            r["kind"] = OP_MCSWAP
-        elif name == "cswap":
-            r["kind"] = OP_MCSWAP
-        elif name == "crz":
-            r["kind"] = OP_MCU1
-            _set_m(r, G.mat1("rz", ins.params))
-        elif name == "cu":
-            r["kind"] = OP_MCU1
-            _set_m(r, G.cu_target(ins.params))
-        elif name in G.CONTROLLED_1Q:
-            r["kind"] = OP_MCU1
-            _set_m(r, G.mat1(G.CONTROLLED_1Q[name], ins.params))
-        elif name in G.CONTROLLED_PHASE:
-            r["kind"] = OP_MCPHASE
-            _set_m(r, [complex(G.CONTROLLED_PHASE[name](ins.params))])
-        elif name == "rzz":
-            r["kind"] = OP_DIAG2
-            _set_m(r, np.diagonal(G.pauli_rot2("z", "z", float(ins.params[0]))))
-        elif name in G.PAULI_ROT_2Q:
-            r["kind"] = OP_U2
-            _set_m(r, G.pauli_rot2(*G.PAULI_ROT_2Q[name], float(ins.params[0])))
-        elif name == "iswap":
-            r["kind"] = OP_U2
-            _set_m(r, G.ISWAP)
-        elif name == "r":
-            r["kind"] = OP_U1
-            _set_m(r, G.r_gate(float(ins.params[0]), float(ins.params[1])))
-        elif name == "mcu":
-            r["kind"] = OP_MCU1 if int(ins.params[0]) == 1 else OP_MCU2
-            _set_m(r, ins.matrix)
-        elif name == "dcx":
+        nq = len(qs)
+        if nq > 8:
+            raise ValueError(f"{name} on {nq} qubits: an op takes at most 8")
+        if name == "dcx":
             # CX(q0 -> q1) then CX(q1 -> q0): two exact permutations
-            r["kind"] = OP_MCX
-            k += 1
-            r2 = recs[k]
-            r2["param"], r2["nq"], r2["kind"] = -1, 2, OP_MCX
-            r2["q"][:2] = (qs[1], qs[0])
-        else:
-            raise ValueError(f"Unsupported instruction: {name}")
-        k += 1
-    return recs[:k]
+            for a, b in ((qs[0], qs[1]), (qs[1], qs[0])):
+                parts += [_HEAD.pack(OP_MCX, 2, a, b, 0, 0, 0, 0, 0, 0, -1, 0), _ZEROS]
+            continue
+        kind, param, m = _lower_one(ins)
+        parts += [_HEAD.pack(kind, nq, *qs, *_NO_QUBITS[8 - nq], param, 0), m]
+        if len(m) < 256:
+            parts.append(_ZEROS[len(m):])
+    return np.frombuffer(bytearray(b"".join(parts)), dtype=OP_DTYPE)
 
 
 def op_u2(q0: int, q1: int, m4: np.ndarray) -> np.ndarray:
