@@ -336,6 +336,7 @@ struct Merger {
       DevOp d;
       std::memset(&d, 0, sizeof(d));
       d.kind = DK_NOISE;
+      if (e.second.kind != QS_OP_DEPOLARIZE) b.pos[7] = 1;
       d.t0 = (uint8_t)e.second.q;
       d.d0 = (uint8_t)e.second.kind;
       d.coef = (uint32_t)e.first;
@@ -345,13 +346,41 @@ struct Merger {
     b.op_end = (int32_t)ops.size();
     blocks.push_back(b);
   }
+
+  // Channels and gates that together are one map of the bins of Q: a header
+  // with the number of blocks behind it, then the channels of groups[0], the
+  // gate plans[0], groups[1], ...  Without gates, a noise block by itself.
+  void add_chain(uint64_t Q, const std::vector<std::vector<std::pair<int, NoiseSite>>>& groups,
+                 const std::vector<qs_plan_s>& plans, size_t ncoef) {
+    if (!blocks.empty() && coef.size() / 2 + ncoef > coef_cap) flush();
+    if (plans.empty()) {
+      if (!groups[0].empty()) add_noise_group(groups[0]);
+      return;
+    }
+    DevBlock b;
+    std::memset(&b, 0, sizeof(b));
+    for (int q = 0; q < n; ++q)
+      if ((Q >> q) & 1) b.pos[b.pos[5]++] = (int8_t)q;
+    b.pos[6] = 1;
+    b.op_begin = b.op_end = (int32_t)ops.size();
+    const size_t at = blocks.size();
+    blocks.push_back(b);
+    for (size_t k = 0; k < groups.size(); ++k) {
+      if (!groups[k].empty()) {
+        add_noise_group(groups[k]);
+        blocks[at].pos[7] |= blocks.back().pos[7];
+      }
+      if (k < plans.size()) add_plan(plans[k]);
+    }
+    blocks[at].pos[4] = (int8_t)(blocks.size() - 1 - at);
+  }
 };
 
 // The circuit's op stream cut into unitary segments; seg_site[s] is the
-// site that follows segment s.  With br (a depolarizing outcome pattern),
-// each depolarizing site becomes its Pauli (or nothing) and only the
-// state-dependent sites cut; without it every site cuts.
-void segment_stream(const qs_op* ops, int nops, const std::vector<NoiseSite>& sites, const std::vector<uint8_t>* br,
+// site that follows segment s.  br is a depolarizing outcome pattern: each
+// depolarizing site becomes its Pauli (or nothing) and only the state-dependent
+// sites cut.
+void segment_stream(const qs_op* ops, int nops, const std::vector<NoiseSite>& sites, const std::vector<uint8_t>& br,
                     std::vector<std::vector<qs_op>>& seg_ops, std::vector<int>& seg_site) {
   seg_ops.assign(1, {});
   seg_site.clear();
@@ -359,8 +388,8 @@ void segment_stream(const qs_op* ops, int nops, const std::vector<NoiseSite>& si
   for (int i = 0; i < nops; ++i) {
     if (k < sites.size() && sites[k].op == i) {
       const NoiseSite& s = sites[k];
-      if (br && s.kind == QS_OP_DEPOLARIZE) {
-        const uint8_t b = (*br)[k];
+      if (s.kind == QS_OP_DEPOLARIZE) {
+        const uint8_t b = br[k];
         if (b) seg_ops.back().push_back(pauli_op(s.q, b));
       } else {
         seg_site.push_back((int)k);
@@ -388,24 +417,8 @@ std::vector<NoiseSite> noise_sites(int n, const qs_op* ops, int nops) {
 
 // The program of a noisy circuit on up to 14 qubits: its unitary segments
 // planned as whole-state passes, consecutive channels grouped into noise
-// blocks between them.  auto_bb: the block width was not fixed by the caller.
-qs_plan_s whole_state_program(int n, const qs_op* ops, int nops, const std::vector<NoiseSite>& sites, int tb, int bb,
-                              bool auto_bb) {
-  std::vector<std::vector<qs_op>> seg;
-  std::vector<int> seg_site;
-  segment_stream(ops, nops, sites, nullptr, seg, seg_site);
-  // channels after (almost) every gate leave segments of one or two gates:
-  // 3-qubit register blocks then beat wider ones (smaller diagonal tables,
-  // so more CTAs per SM; measured 204 k vs 182 k trajectories/s on a
-  // 12-qubit, 840-channel circuit)
-  {
-    size_t nonempty = 0, gates = 0;
-    for (const auto& sg : seg) {
-      nonempty += !sg.empty();
-      gates += sg.size();
-    }
-    if (auto_bb && nonempty && gates <= 4 * nonempty) bb = std::min(bb, 3);
-  }
+// blocks between them.
+qs_plan_s whole_state_program(int n, const qs_op* ops, int nops, const std::vector<NoiseSite>& sites, int tb, int bb) {
   const size_t smem_left = 200 * 1024 - (8ull << n) - 2 * 128 * sizeof(uint64_t) - 16 * sizeof(int) - 16;
   Merger m;
   m.n = n;
@@ -413,36 +426,142 @@ qs_plan_s whole_state_program(int n, const qs_op* ops, int nops, const std::vect
   m.coef_cap = std::min<size_t>(8192, smem_left / sizeof(float2));
   m.out.n_qubits = n;
   double flops = 0;
-  // consecutive channels (no gate between) share a block while they touch
-  // at most kGroupQubits qubits and number at most kGroupOps
-  constexpr int kGroupQubits = 4, kGroupOps = 32;
-  std::vector<std::pair<int, NoiseSite>> group;
-  auto group_qubits = [&](int extra) {
-    std::vector<int> qs;
-    for (const auto& e : group)
-      if (std::find(qs.begin(), qs.end(), e.second.q) == qs.end()) qs.push_back(e.second.q);
-    if (extra >= 0 && std::find(qs.begin(), qs.end(), extra) == qs.end()) qs.push_back(extra);
-    return (int)qs.size();
+  auto plan_of = [&](const std::vector<qs_op>& g) {
+    qs_plan_s p;
+    qs_build_plan(n, g.data(), (int)g.size(), tb, &p, bb);
+    return p;
   };
-  auto flush_group = [&]() {
-    if (!group.empty()) m.add_noise_group(group);
-    group.clear();
+  // Scheduling: gates and channels keep their order on every qubit and the
+  // channels their order among themselves (a gate commutes with a channel on
+  // other qubits, and does not change its branch probabilities).
+  //   * A chain is the next channels, and the permutations and diagonals in front
+  //     of them, while they touch at most kGroupQubits qubits: one map in the
+  //     kernel (noise_block).
+  //   * Where a dense gate is in front of the next channel, a unitary segment:
+  //     every gate that can run now and that a dense gate among them needs.
+  constexpr int kGroupQubits = 4, kGroupOps = 32, kGroupGates = 64;
+  std::vector<int> site_of(nops, -1);
+  for (size_t k = 0; k < sites.size(); ++k) site_of[sites[k].op] = (int)k;
+  std::vector<std::vector<int>> on(n);
+  for (int i = 0; i < nops; ++i)
+    for (int q = 0; q < ops[i].nq; ++q) {
+      qs_check_qubit(ops[i].q[q], n, "op");
+      on[ops[i].q[q]].push_back(i);
+    }
+  std::vector<size_t> head(n, 0);
+  std::vector<char> no_chain(nops, 0);
+  auto front = [&](int i, const std::vector<size_t>& at) {
+    for (int q = 0; q < ops[i].nq; ++q)
+      if (on[ops[i].q[q]][at[ops[i].q[q]]] != i) return false;
+    return true;
   };
-  for (size_t s = 0; s < seg.size(); ++s) {
-    if (!seg[s].empty()) {
-      flush_group();
-      qs_plan_s p;
-      qs_build_plan(n, seg[s].data(), (int)seg[s].size(), tb, &p, bb);
-      m.add_plan(p);
-      flops += p.info.flops;
+  auto advance = [&](int i, std::vector<size_t>& at) {
+    for (int q = 0; q < ops[i].nq; ++q) ++at[ops[i].q[q]];
+  };
+  auto qubits = [&](int i) {
+    uint64_t m = 0;
+    for (int q = 0; q < ops[i].nq; ++q) m |= 1ull << ops[i].q[q];
+    return m;
+  };
+  auto maps_bins = [&](int i) {
+    const int k = ops[i].kind;
+    return !no_chain[i] && (k == QS_OP_MCX || k == QS_OP_Y || k == QS_OP_MCPHASE || k == QS_OP_DIAG1 ||
+                            k == QS_OP_DIAG2 || k == QS_OP_MCSWAP || k == QS_OP_RZ);
+  };
+  // every gate that can run before another channel, in an order that respects the circuit's
+  auto closure = [&]() {
+    std::vector<int> got;
+    std::vector<size_t> at(head);
+    for (bool more = true; more;) {
+      more = false;
+      for (int q = 0; q < n; ++q)
+        while (at[q] < on[q].size() && site_of[on[q][at[q]]] < 0 && front(on[q][at[q]], at)) {
+          const int i = on[q][at[q]];
+          advance(i, at);
+          got.push_back(i);
+          more = true;
+        }
     }
-    if (s < seg_site.size()) {
-      const NoiseSite& ns = sites[seg_site[s]];
-      if ((int)group.size() >= kGroupOps || group_qubits(ns.q) > kGroupQubits) flush_group();
-      group.emplace_back(seg_site[s], ns);
+    std::sort(got.begin(), got.end());
+    return got;
+  };
+  auto segment = [&](const std::vector<int>& gates) {
+    std::vector<qs_op> seg;
+    for (int i : gates) {
+      seg.push_back(ops[i]);
+      advance(i, head);
     }
+    const qs_plan_s p = plan_of(seg);
+    m.add_plan(p);
+    flops += p.info.flops;
+  };
+  size_t next = 0;   // channel
+  while (next < sites.size()) {
+    // a chain
+    std::vector<std::vector<std::pair<int, NoiseSite>>> groups;   // channels, each group in front of a gate
+    std::vector<qs_plan_s> plans;
+    uint64_t Q = 0;
+    size_t ncoef = 0;
+    int nch = 0;
+    groups.emplace_back();
+    while (next < sites.size()) {
+      int i = sites[next].op;
+      if (front(i, head)) {
+        if (nch >= kGroupOps || __builtin_popcountll(Q | qubits(i)) > kGroupQubits) break;
+        Q |= qubits(i);
+        groups.back().emplace_back((int)next, sites[next]);
+        advance(i, head);
+        ++nch;
+        ++next;
+        continue;
+      }
+      // the gate that has to run first (channels before this one are done)
+      for (bool found = false; !found;) {
+        found = true;
+        for (int q = 0; q < ops[i].nq && found; ++q) {
+          const int j = on[ops[i].q[q]][head[ops[i].q[q]]];
+          if (j != i) { i = j; found = false; }
+        }
+      }
+      if (!maps_bins(i) || (int)plans.size() >= kGroupGates || __builtin_popcountll(Q | qubits(i)) > kGroupQubits) break;
+      qs_plan_s p = plan_of({ops[i]});
+      bool ok = p.pass_offsets.size() <= 1;
+      for (size_t j = 0; ok && j < p.pass_offsets.size(); ++j) {
+        const auto* hdr = reinterpret_cast<const DevPass*>(p.blob.data() + p.pass_offsets[j]);
+        const auto* pb = reinterpret_cast<const DevBlock*>(reinterpret_cast<const char*>(hdr) + hdr->block_off);
+        const auto* po = reinterpret_cast<const DevOp*>(reinterpret_cast<const char*>(hdr) + hdr->op_off);
+        ok = hdr->nblocks == 1 && ncoef + hdr->ncoef <= m.coef_cap;
+        for (int o = pb[0].op_begin; ok && o < pb[0].op_end; ++o)
+          ok = po[o].kind == DK_X || po[o].kind == DK_Y || po[o].kind == DK_SWAP || po[o].kind == DK_DTAB;
+        ncoef += hdr->ncoef;
+      }
+      if (!ok) {
+        no_chain[i] = 1;   // a gate of a segment from now on
+        break;
+      }
+      Q |= qubits(i);
+      plans.push_back(std::move(p));
+      groups.emplace_back();
+      advance(i, head);
+    }
+    if (nch || !plans.empty()) {
+      m.add_chain(Q, groups, plans, ncoef);
+      continue;
+    }
+    const std::vector<int> all = closure();
+    std::vector<int> gates;
+    uint64_t needed = 0;
+    for (size_t k = all.size(); k-- > 0;) {
+      const uint64_t qs = qubits(all[k]);
+      if (maps_bins(all[k]) && !(qs & needed)) continue;
+      needed |= qs;
+      gates.push_back(all[k]);
+    }
+    std::reverse(gates.begin(), gates.end());
+    segment(gates.empty() ? all : gates);
   }
-  flush_group();
+  const std::vector<int> rest = closure();
+  if (!rest.empty()) segment(rest);
   m.flush(true);
   m.out.info.flops = flops;
   return std::move(m.out);
@@ -493,7 +612,7 @@ int qs_noise_program(int n, const qs_op* ops, int nops, int block_bits, void* ou
   QS_CHECK_ARG(nops >= 0 && (nops == 0 || ops), "ops pointer is null");
   QS_CHECK_ARG(block_bits == 0 || (block_bits >= 2 && block_bits <= 5), "block_bits must be 0 (auto) or in [2, 5]");
   const std::vector<NoiseSite> sites = noise_sites(n, ops, nops);
-  const qs_plan_s p = whole_state_program(n, ops, nops, sites, 13, block_bits ? block_bits : 4, block_bits == 0);
+  const qs_plan_s p = whole_state_program(n, ops, nops, sites, 13, block_bits ? block_bits : 4);
   *needed = p.blob.size();
   if (out && cap >= p.blob.size() && !p.blob.empty()) std::memcpy(out, p.blob.data(), p.blob.size());
   QS_API_END(h)
@@ -524,7 +643,7 @@ int qs_noise_trajectories(qs_handle_t h, int n, const qs_op* ops, int nops, int 
     // one whole-state program with a noise block per channel group, shared
     // by all trajectories; one CTA per trajectory
     std::vector<qs_plan_s> progs(1);
-    progs[0] = whole_state_program(n, ops, nops, sites, tb, bb, h->block_bits == 0);
+    progs[0] = whole_state_program(n, ops, nops, sites, tb, bb);
     std::vector<BatchUnit> units(n_traj);
     for (int t = 0; t < n_traj; ++t)
       units[t] = BatchUnit{0, (uint64_t)t * N, seeds[t], want_br ? d_br + (size_t)t * nn : nullptr};
@@ -557,7 +676,7 @@ int qs_noise_trajectories(qs_handle_t h, int n, const qs_op* ops, int nops, int 
     std::vector<std::vector<std::vector<qs_op>>> seg_of(patterns.size());
     std::vector<int> seg_site;
     for (size_t pi = 0; pi < patterns.size(); ++pi)
-      segment_stream(ops, nops, sites, &patterns[pi], seg_of[pi], seg_site);
+      segment_stream(ops, nops, sites, patterns[pi], seg_of[pi], seg_site);
     const size_t nseg = seg_site.size() + 1;
     bool need_init = false;
     for (int t = 0; t < n_traj; ++t) need_init |= seg_of[traj_pattern[t]][0].empty();

@@ -464,18 +464,26 @@ __device__ __forceinline__ void run_ops(float2 (&v)[1 << R], const DevOp* __rest
 //   Z: c = +1 / -1            no jump: c = r / sqrt(1-g) r, r = 1/sqrt(S0 + (1-g) S1)
 //   damping jump: m = q, c = 1/sqrt(S1) / 0      dephasing jump: c = 0 / 1/sqrt(S1)
 // (E1 of damping is [[0, sqrt g], [0, 0]], of dephasing [[0, 0], [0, sqrt l]],
-// each renormalised exactly).  The form is closed under composition
-// (C'(b) = c(b) C(b ^ m), M' = M ^ m), and so is the bin histogram of |a|^2
-// (H'(b) = |c(b)|^2 H(b ^ m)).  So the block takes one histogram sweep (FP32
-// squares summed in FP64; only when a damping or dephasing channel needs
-// P(q=1)), decides every branch in order from the running histogram in FP64
-// (damping / dephasing: jump when u < p1 = g S1 / (S0 + S1); depolarizing:
-// the reference's ranges), and applies the composed map in one sweep
-// (factors rounded to FP32 once).  Q is ascending (bin bit j = qubit Q[j]).
+// each renormalised exactly).  X, Y, SWAP, their controlled forms and diagonal
+// gates on Q have the same form with a permutation p of the bins for the flip,
+// so a chain (a header block with the number of blocks in pos[4], then noise
+// blocks and blocks of such gates, all within the header's Q) is one map:
+// C'(b) = c(b) C(p(b)), source'(b) = source(p(b)), and the bin histogram of
+// |a|^2 follows it (H'(b) = |c(b)|^2 H(p(b))).  A chain (or a noise block by
+// itself) takes one histogram sweep (FP32 squares summed in FP64; only when a
+// damping or dephasing channel needs P(q=1)), decides every branch in order from
+// the running histogram in FP64 (damping / dephasing: jump when u < p1 = g S1 /
+// (S0 + S1); depolarizing: the reference's ranges), and applies the composed map
+// in one sweep (factors rounded to FP32 once).  Q is ascending (bin bit j =
+// qubit Q[j]).
+//
+// Bound by the decisions' serial FP64 chain and by issue.  1024 trajectories of
+// 12 qubits, 236 gates, 840 channels: 1.6 ms in 32 register blocks and 48
+// chains; 5.47 ms when every gate was a register block followed by a noise block.
 struct NoiseSmem {
   double red[16 * 16];  // per-warp bin sums (at most 16 warps per CTA)
   float2 C[16];        // composed factor per bin
-  uint32_t M;          // composed flip mask over the bins (bit j = qubit Q[j])
+  uint32_t src[16];    // the bin that a bin's amplitudes come from
   uint32_t identity;   // 1: the composed map is the identity
 };
 
@@ -484,13 +492,12 @@ struct NoiseSmem {
 // phys(base | off(b)) = phys(base) ^ phys(off(b)).
 template <int NQ>
 __device__ __forceinline__ void bin_offsets(const int (&Q)[4], uint32_t (&poff)[1 << NQ]) {
+  poff[0] = 0;
 #pragma unroll
-  for (int b = 0; b < (1 << NQ); ++b) {
-    uint32_t off = 0;
+  for (int j = 0; j < NQ; ++j) {
+    const uint32_t p = phys(1u << Q[j]);
 #pragma unroll
-    for (int j = 0; j < NQ; ++j)
-      if ((b >> j) & 1) off |= 1u << Q[j];
-    poff[b] = phys(off);
+    for (int b = 0; b < (1 << j); ++b) poff[b | (1 << j)] = poff[b] ^ p;
   }
 }
 
@@ -515,57 +522,82 @@ __device__ __forceinline__ void noise_hist(const float2* tile, uint32_t N, const
       acc[b] += (double)fmaf(a.x, a.x, __fmul_rn(a.y, a.y));
     }
   }
+  // the butterfly over the lanes, each round passing half of the bins on
+  const int lane = threadIdx.x & 31;
+  int bin = 0;
 #pragma unroll
-  for (int b = 0; b < NB; ++b) {
-    double v = acc[b];
+  for (int o = 16, h = NB / 2; o > 0; o >>= 1, h >>= 1) {
+    const bool up = lane & o;
+    if (h > 0) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) red[(threadIdx.x >> 5) * 16 + b] = v;
+      for (int b = 0; b < h; ++b) {
+        const double keep = up ? acc[b + h] : acc[b], send = up ? acc[b] : acc[b + h];
+        acc[b] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+      if (up) bin += h;
+    } else {
+      acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+    }
   }
+  if ((lane & (32 / NB - 1)) == 0) red[(threadIdx.x >> 5) * 16 + bin] = acc[0];
 }
 
-// a'(base | off(b)) = C[b] * a(base | off(b ^ M)) over every base.
+// a'(base | off(b)) = C[b] * a(base | off(src[b])) over every base.
 template <int NQ>
 __device__ __forceinline__ void noise_apply(float2* tile, uint32_t N, const int (&Q)[4], const NoiseSmem* sm) {
   constexpr int NB = 1 << NQ;
-  uint32_t poff[NB];
+  uint32_t poff[NB], psrc[NB];
   bin_offsets<NQ>(Q, poff);
-  const uint32_t M = sm->M;
-  float2 Cv[NB], Cm[NB];  // C[b] and C[b ^ M]
 #pragma unroll
-  for (int b = 0; b < NB; ++b) { Cv[b] = sm->C[b]; Cm[b] = sm->C[b ^ M]; }
+  for (int b = 0; b < NB; ++b) {
+    const uint32_t x = sm->src[b];
+    psrc[b] = 0;
+#pragma unroll
+    for (int j = 0; j < NQ; ++j)
+      if ((x >> j) & 1) psrc[b] ^= poff[1 << j];
+  }
   for (uint32_t r = threadIdx.x; r < (N >> NQ); r += blockDim.x) {
     uint32_t base = r;
 #pragma unroll
     for (int j = 0; j < NQ; ++j) base = (uint32_t)insert_zero(base, Q[j]);
     const uint32_t pb = phys(base);
-    if (M == 0) {
+    float2 v[NB];
 #pragma unroll
-      for (int b = 0; b < NB; ++b) {
-        float2& a = tile[pb ^ poff[b]];
-        a = cmul(a, Cv[b]);
-      }
-    } else {
+    for (int b = 0; b < NB; ++b) v[b] = tile[pb ^ psrc[b]];
 #pragma unroll
-      for (int b = 0; b < NB; ++b) {
-        const int b2 = b ^ (int)M;
-        if (b2 < b) continue;
-        float2& ai = tile[pb ^ poff[b]];
-        float2& aj = tile[pb ^ poff[b2]];
-        const float2 vi = ai, vj = aj;
-        ai = cmul(vj, Cv[b]);
-        aj = cmul(vi, Cm[b]);
-      }
-    }
+    for (int b = 0; b < NB; ++b) tile[pb ^ poff[b]] = cmul(v[b], sm->C[b]);
   }
 }
 
-// Warp 0: the branch of every channel of the block, in order, and the
-// composed map.  Lane b < 2^nq holds bin b (its histogram entry and factor);
-// sums over bins are xor butterflies, so every lane gets the same bits.  A
-// branch's factor c(b) takes one of two values by bit q of the bin (lo for
-// bit clear, hi for bit set).
-__device__ __noinline__ void noise_decide(const DevOp* __restrict__ ops, int ob, int oe, const int (&Q)[4], int nq,
+// The factor of a merged diagonal (op_dtab's layout) on register index j and
+// group index gidx.
+__device__ __forceinline__ double2 dtab_factor(const DevOp& op, const float2* __restrict__ c, int R, uint32_t j,
+                                               uint64_t gidx) {
+  double2 f = make_double2(1.0, 0.0);
+  auto times = [&](float2 w) {
+    f = make_double2(f.x * w.x - f.y * w.y, f.x * w.y + f.y * w.x);
+  };
+  const float2* p = c;
+  if (op.rc & 1) {
+    times(c[j]);
+    p += 1 << R;
+  }
+  for (int k = 0; k < op.t0; ++k, p += 2)
+    if ((gidx & bits64(p[0])) == bits64(p[0])) times(p[1]);
+  for (int k = 0; k < op.t1; ++k, p += 2)
+    if ((gidx & bits64(p[1])) == bits64(p[1]) && ((__float_as_uint(p[0].x) >> j) & 1u)) times(make_float2(-1.f, 0.f));
+  for (int k = 0; k < op.d0; ++k, p += 3)
+    if ((gidx & bits64(p[1])) == bits64(p[1]) && ((__float_as_uint(p[0].x) >> j) & 1u)) times(p[2]);
+  return f;
+}
+
+// Warp 0: the branch of every channel of the chain, in order, and the
+// composed map.  Lane b < 2^nq holds bin b (its histogram entry, factor and
+// source); sums over bins are xor butterflies, so every lane gets the same
+// bits.  A branch's factor c(b) takes one of two values by bit q of the bin (lo
+// for bit clear, hi for bit set).
+__device__ __noinline__ void noise_decide(const DevBlock* __restrict__ blks, int nblk, const DevOp* __restrict__ ops,
+                                         const float2* __restrict__ coef, int R, const int (&Q)[4], int nq,
                                          bool have_h, int nw, uint64_t seed, uint8_t* nb, NoiseSmem* sm) {
   const int lane = threadIdx.x & 31;
   const int NB = 1 << nq;
@@ -573,73 +605,140 @@ __device__ __noinline__ void noise_decide(const DevOp* __restrict__ ops, int ob,
   double H = 0.0, Cr = 1.0, Ci = 0.0;
   if (have_h && mine)
     for (int w = 0; w < nw; ++w) H += sm->red[w * 16 + lane];
-  uint32_t mb = 0;
+  int src = lane;
   bool ident = true;
-  for (int o = ob; o < oe; ++o) {
-    const DevOp op = ops[o];
+  uint64_t at = 0;   // the bin's bits of the amplitude index
+  for (int j = 0; j < nq; ++j)
+    if ((lane >> j) & 1) at |= 1ull << Q[j];
+  auto bin_bit = [&](int q) {
     int j = 0;
-    while (j < nq - 1 && Q[j] != op.t0) ++j;
-    const int bit = 1 << j;
-    const bool set = (lane & bit) != 0;
-    const double g = __longlong_as_double((long long)op.gc);
-    const double u = qs_seed_uniform_at(seed, op.coef);
-    int m = 0;
-    double cr = 1.0, ci = 0.0;
-    if (op.d0 == QS_OP_DEPOLARIZE) {
-      const int br = qs_depol_branch(g, u);
-      if (lane == 0 && nb) nb[op.coef] = (uint8_t)br;
-      if (br == 0) continue;
-      if (br == 1) m = bit;
-      else if (br == 2) { m = bit; cr = 0.0; ci = set ? 1.0 : -1.0; }
-      else cr = set ? -1.0 : 1.0;
-    } else {
-      double s1 = set ? H : 0.0, s0 = set ? 0.0 : H;
-#pragma unroll
-      for (int x = 1; x < 16; x <<= 1) {
-        s0 += __shfl_xor_sync(0xffffffffu, s0, x);
-        s1 += __shfl_xor_sync(0xffffffffu, s1, x);
+    while (j < nq - 1 && Q[j] != q) ++j;
+    return 1 << j;
+  };
+  // the chain's channels (at most 32), one per lane: what does not depend on the
+  // state is worked out at once
+  int info = 0;        // kind (3: none), bit of the bin << 2, depolarizing branch << 6
+  double cg = 0.0, cu = 0.0, csq = 0.0;
+  uint32_t cslot = 0;
+  {
+    int first = 0;
+    for (int k = 0; k < nblk; ++k) {
+      if (!blks[k].pos[6]) continue;
+      const int o = blks[k].op_begin + lane - first;
+      if (o >= blks[k].op_begin && o < blks[k].op_end) {
+        const DevOp op = ops[o];
+        cg = __longlong_as_double((long long)op.gc);
+        cu = qs_seed_uniform_at(seed, op.coef);
+        csq = sqrt(1.0 - cg);
+        cslot = op.coef;
+        info = (op.d0 == QS_OP_DEPOLARIZE ? 0 : op.d0 == QS_OP_AMP_DAMP ? 1 : 2) | bin_bit(op.t0) << 2;
+        if (op.d0 == QS_OP_DEPOLARIZE) {
+          const int br = qs_depol_branch(cg, cu);
+          info |= br << 6;
+          if (nb) nb[cslot] = (uint8_t)br;
+        }
       }
-      const double S0 = s0, S1 = s1;
-      const double p1 = g * S1 / (S0 + S1);
-      // the kept branch has norm^2 keep; a branch of zero weight is never taken
-      const double keep = S0 + (1.0 - g) * S1;
-      const bool jump = S1 > 0.0 && (u < p1 || !(keep > 0.0));
-      if (lane == 0 && nb) nb[op.coef] = jump ? 1 : 0;
-      if (!jump) {
-        const double r = 1.0 / sqrt(keep);
-        cr = set ? sqrt(1.0 - g) * r : r;
-      } else if (op.d0 == QS_OP_AMP_DAMP) {
-        m = bit;
-        cr = set ? 0.0 : 1.0 / sqrt(S1);
-      } else {
-        cr = set ? 1.0 / sqrt(S1) : 0.0;
-      }
+      first += blks[k].op_end - blks[k].op_begin;
     }
-    ident = false;
-    // C'(b) = c(b) C(b ^ m), H'(b) = |c(b)|^2 H(b ^ m)
-    const double xr = __shfl_xor_sync(0xffffffffu, Cr, m), xi = __shfl_xor_sync(0xffffffffu, Ci, m);
-    const double xh = __shfl_xor_sync(0xffffffffu, H, m);
+  }
+  int chan = 0;
+  // a'(b) = c(b) a(p(b)) on top of the map so far
+  auto step = [&](int p, double cr, double ci) {
+    const double xr = __shfl_sync(0xffffffffu, Cr, p), xi = __shfl_sync(0xffffffffu, Ci, p);
+    const double xh = __shfl_sync(0xffffffffu, H, p);
+    src = __shfl_sync(0xffffffffu, src, p);
     Cr = cr * xr - ci * xi;
     Ci = cr * xi + ci * xr;
     H = (cr * cr + ci * ci) * xh;
-    mb ^= (uint32_t)m;
+    ident = false;
+  };
+  for (int k = 0; k < nblk; ++k) {
+    const DevBlock blk = blks[k];
+    if (!blk.pos[6]) {   // gates that only permute the bins or multiply them
+      uint32_t j = 0;
+      uint64_t g = at;
+      for (int r = 0; r < R; ++r) {
+        j |= (uint32_t)((at >> blk.pos[r]) & 1) << r;
+        g &= ~(1ull << blk.pos[r]);
+      }
+      for (int o = blk.op_begin; o < blk.op_end; ++o) {
+        const DevOp op = ops[o];
+        if (op.kind == DK_DTAB) {
+          const double2 f = dtab_factor(op, coef + op.coef, R, j, g);
+          step(lane, f.x, f.y);
+          continue;
+        }
+        const bool on = (g & op.gc) == op.gc && (j & op.rc) == op.rc;
+        const int bit = bin_bit(blk.pos[op.t0]);
+        if (op.kind == DK_SWAP) {
+          const int bit1 = bin_bit(blk.pos[op.t1]);
+          step(on && !(lane & bit) != !(lane & bit1) ? lane ^ bit ^ bit1 : lane, 1.0, 0.0);
+        } else if (op.kind == DK_Y) {
+          step(on ? lane ^ bit : lane, on ? 0.0 : 1.0, on ? (lane & bit ? 1.0 : -1.0) : 0.0);
+        } else {  // DK_X
+          step(on ? lane ^ bit : lane, 1.0, 0.0);
+        }
+      }
+      continue;
+    }
+    for (int o = blk.op_begin; o < blk.op_end; ++o, ++chan) {
+      const int ch = __shfl_sync(0xffffffffu, info, chan);
+      const double g = __shfl_sync(0xffffffffu, cg, chan), u = __shfl_sync(0xffffffffu, cu, chan);
+      const double sq = __shfl_sync(0xffffffffu, csq, chan);
+      const int bit = (ch >> 2) & 15;
+      const bool set = (lane & bit) != 0;
+      int m = 0;
+      double cr = 1.0, ci = 0.0;
+      if ((ch & 3) == 0) {
+        const int br = ch >> 6;
+        if (br == 0) continue;
+        if (br == 1) m = bit;
+        else if (br == 2) { m = bit; cr = 0.0; ci = set ? 1.0 : -1.0; }
+        else cr = set ? -1.0 : 1.0;
+      } else {
+        double s1 = set ? H : 0.0, s0 = set ? 0.0 : H;
+        for (int x = 1; x < NB; x <<= 1) {
+          s0 += __shfl_xor_sync(0xffffffffu, s0, x);
+          s1 += __shfl_xor_sync(0xffffffffu, s1, x);
+        }
+        // lanes past the bins hold zeros: the totals of lane 0's bins
+        const double S0 = __shfl_sync(0xffffffffu, s0, 0), S1 = __shfl_sync(0xffffffffu, s1, 0);
+        // the kept branch has norm^2 keep; a branch of zero weight is never
+        // taken; u < p1 = g S1 / (S0 + S1) without the division
+        const double keep = S0 + (1.0 - g) * S1;
+        const bool jump = S1 > 0.0 && (u * (S0 + S1) < g * S1 || !(keep > 0.0));
+        if (lane == chan && nb) nb[cslot] = jump ? 1 : 0;
+        if (!jump) {
+          const double r = rsqrt(keep);
+          cr = set ? sq * r : r;
+        } else if ((ch & 3) == 1) {
+          m = bit;
+          cr = set ? 0.0 : rsqrt(S1);
+        } else {
+          cr = set ? rsqrt(S1) : 0.0;
+        }
+      }
+      step(lane ^ m, cr, ci);
+    }
   }
-  if (mine) sm->C[lane] = make_float2((float)Cr, (float)Ci);
-  if (lane == 0) {
-    sm->M = mb;
-    sm->identity = ident ? 1u : 0u;
+  if (mine) {
+    sm->C[lane] = make_float2((float)Cr, (float)Ci);
+    sm->src[lane] = (uint32_t)src;
   }
+  if (lane == 0) sm->identity = ident ? 1u : 0u;
 }
 
-__device__ __noinline__ void noise_block(float2* tile, int T, const DevBlock blk, const DevOp* __restrict__ ops,
+// A noise block (nblk = 1, blks its own record) or a chain: head's Q, the
+// blocks behind it.
+__device__ __noinline__ void noise_block(float2* tile, int T, const DevBlock head, const DevBlock* __restrict__ blks,
+                                        int nblk, const DevOp* __restrict__ ops, const float2* __restrict__ coef, int R,
                                         uint64_t seed, uint8_t* nb, NoiseSmem* sm) {
   const uint32_t N = 1u << T;
-  const int nq = blk.pos[5];
+  const int nq = head.pos[5];
   int Q[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) Q[j] = blk.pos[j];
-  bool have_h = false;
-  for (int o = blk.op_begin; o < blk.op_end; ++o) have_h |= ops[o].d0 != QS_OP_DEPOLARIZE;
+  for (int j = 0; j < 4; ++j) Q[j] = head.pos[j];
+  const bool have_h = head.pos[7] != 0;   // a channel needs P(q = 1)
   if (have_h) {
     switch (nq) {
       case 1: noise_hist<1>(tile, N, Q, sm->red); break;
@@ -650,7 +749,7 @@ __device__ __noinline__ void noise_block(float2* tile, int T, const DevBlock blk
     __syncthreads();
   }
   if (threadIdx.x < 32)
-    noise_decide(ops, blk.op_begin, blk.op_end, Q, nq, have_h, (int)(blockDim.x >> 5), seed, nb, sm);
+    noise_decide(blks, nblk, ops, coef, R, Q, nq, have_h, (int)(blockDim.x >> 5), seed, nb, sm);
   __syncthreads();
   if (sm->identity) return;
   switch (nq) {
@@ -820,8 +919,11 @@ k_pass(float2* __restrict__ base_state, PassItem single, const PassItem* __restr
     for (int b = 0; b < nblocks; ++b) {
       const DevBlock blk = blocks[b];
       if (blk.pos[6]) {  // noise block (only in programs whose tile is the whole state)
-        noise_block(tile, T, blk, ops, I.noise_seed, I.noise_branch, &s_noise);
+        const int chain = blk.pos[4];
+        noise_block(tile, T, blk, blocks + b + (chain ? 1 : 0), chain ? chain : 1, ops, s_coef, R, I.noise_seed,
+                    I.noise_branch, &s_noise);
         __syncthreads();
+        b += chain;
         continue;
       }
       register_block<R, TWO>(tile, blk, ops, s_coef, ngroups, gbase, dep_lo, dep_hi);
