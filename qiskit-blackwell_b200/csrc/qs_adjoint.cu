@@ -227,14 +227,6 @@ struct PassArg {
 
 __device__ __forceinline__ float2 conjf2(float2 a) { return make_float2(a.x, -a.y); }
 
-// The column of position k before any CNOT, in elements.  Its low four bits
-// choose the banks: powers of a primitive element of GF(16), so that four
-// neighbours span them all, also after chains of CNOTs (sums of neighbours are
-// such powers again).
-__host__ __device__ constexpr uint32_t adj_first_col(int k) {
-  return (1u << k) | (uint32_t)((0xE7A5BC638421ull >> (4 * k)) & 15);
-}
-
 // Sums v[0..N) over the warp; returns the index of the total that this lane's
 // v[0] then holds, -1 if none.  Each round passes half of the values on, so
 // nine cost 12 exchanges instead of 45.
@@ -279,21 +271,6 @@ __device__ __forceinline__ void adj_gate(float2 (&re)[8], float2 (&im)[8], const
     im[i] = __ffma2_rn(g1y, r1, __ffma2_rn(g1x, i1, __ffma2_rn(g0y, r0, __fmul2_rn(g0x, i0))));
     re[k] = __ffma2_rn(m3y, i1, __ffma2_rn(g3x, r1, __ffma2_rn(m2y, i0, __fmul2_rn(g2x, r0))));
     im[k] = __ffma2_rn(g3y, r1, __ffma2_rn(g3x, i1, __ffma2_rn(g2y, r0, __fmul2_rn(g2x, i0))));
-  }
-}
-
-// U on the pairs of register bit J of 16 amplitudes.
-template <int J>
-__device__ __forceinline__ void adj_gate(float2 (&a)[16], const float4* __restrict__ U) {
-  const float4 A = U[0], B = U[1];
-  const float2 g0 = make_float2(A.x, A.y), g1 = make_float2(A.z, A.w), g2 = make_float2(B.x, B.y),
-               g3 = make_float2(B.z, B.w);
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int i = ((q >> J) << (J + 1)) | (q & ((1 << J) - 1)), k = i | (1 << J);
-    const float2 a0 = a[i], a1 = a[k];
-    a[i] = cfma2(g0, a0, g1, a1);
-    a[k] = cfma2(g2, a0, g3, a1);
   }
 }
 
@@ -376,7 +353,7 @@ __global__ void __launch_bounds__(kThreads, FWD ? 3 : 2)
   };
   auto addr = [&](uint32_t i) -> uint32_t { return map_lo[i & 63] ^ map_hi[i >> 6]; };
   if (tid < kChunks) step_put(0, step_chunk(P.gb));
-  map_build(0, 1, [&](int k) { return adj_first_col(k) * kElem; });
+  map_build(0, 1, [&](int k) { return tile_col(k) * kElem; });
   uint64_t gbase = tile;
   for (int k = 0; k < P.bits; ++k) gbase = insert_zero(gbase, P.S[k]);
   __syncthreads();
@@ -444,10 +421,10 @@ __global__ void __launch_bounds__(kThreads, FWD ? 3 : 2)
           float2 w[16];
 #pragma unroll
           for (int r = 0; r < 16; ++r) w[r] = el(A ^ off[r]);
-          if (G.gates & 1) adj_gate<0>(w, U);
-          if (G.gates & 2) adj_gate<1>(w, U + 2);
-          if (G.gates & 4) adj_gate<2>(w, U + 4);
-          if (G.gates & 8) adj_gate<3>(w, U + 6);
+          if (G.gates & 1) gate_on_bit<0>(w, U);
+          if (G.gates & 2) gate_on_bit<1>(w, U + 2);
+          if (G.gates & 4) gate_on_bit<2>(w, U + 4);
+          if (G.gates & 8) gate_on_bit<3>(w, U + 6);
 #pragma unroll
           for (int r = 0; r < 16; ++r) el(A ^ off[r]) = w[r];
         } else {
@@ -829,7 +806,7 @@ struct AdjPlan {
     int k = 0;
     for (int q = 0; q < n; ++q)
       if ((S >> q) & 1) { P.S[k] = q; pos[q] = k++; }
-    for (int j = 0; j < T; ++j) col[j] = adj_first_col(j);
+    for (int j = 0; j < T; ++j) col[j] = tile_col(j);
     cst = 0;
     out.clear();
     P.gb = (int)steps.size();

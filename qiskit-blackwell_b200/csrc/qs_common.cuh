@@ -133,6 +133,31 @@ __device__ __forceinline__ float2 cfma4(const float2* g, float2 a0, float2 a1, f
   return make_float2(re, im);
 }
 
+// ---------------------------------------------- tiles in shared memory ----
+// Amplitude i of a 2^12-amplitude tile lies at the XOR of the columns of its
+// set bits (in elements).  A column's low four bits choose the banks: powers of a
+// primitive element of GF(16), so that four neighbours span them all, also
+// after chains of CNOTs (sums of neighbours are such powers again).
+__host__ __device__ constexpr uint32_t tile_col(int k) {
+  return k < 4 ? 1u << k : (1u << k) | (uint32_t)((0xE7A5BC638421ull >> (4 * k)) & 15);
+}
+
+// A 2x2 matrix (two 16-byte rows) on the pairs of register bit J of 16
+// amplitudes, as FMA chains.
+template <int J>
+__device__ __forceinline__ void gate_on_bit(float2 (&a)[16], const float4* __restrict__ U) {
+  const float4 A = U[0], B = U[1];
+  const float2 g0 = make_float2(A.x, A.y), g1 = make_float2(A.z, A.w), g2 = make_float2(B.x, B.y),
+               g3 = make_float2(B.z, B.w);
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int i = ((q >> J) << (J + 1)) | (q & ((1 << J) - 1)), k = i | (1 << J);
+    const float2 a0 = a[i], a1 = a[k];
+    a[i] = cfma2(g0, a0, g1, a1);
+    a[k] = cfma2(g2, a0, g3, a1);
+  }
+}
+
 // ------------------------------------------------------ vector memory -----
 __device__ __forceinline__ float4 ld4(const float2* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void st4(float2* p, float2 a, float2 b) {

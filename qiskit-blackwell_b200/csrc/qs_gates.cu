@@ -94,21 +94,21 @@ __global__ void k_1q_tn(float2* __restrict__ s, uint64_t nitems, int t, G2 G0, c
 
 // K <= 12 single-qubit gates whose matrices and targets are device arrays,
 // applied in one launch (the device-tensor form of apply_gates_fused: no host
-// copy of the gates, no stream synchronisation).  Each CTA stages tiles of
+// copy of the gates, no stream synchronisation).  A CTA stages a tile of
 // 2^T amplitudes (T = min(n, 12)) whose qubits are the gates' distinct
 // targets and the lowest other qubits, applies the gates to the tile in
 // shared memory as an FMA chain per output (each FMA rounds once; the
 // single-gate kernels' compensated Dot2 costs four times the arithmetic),
 // and writes the tile back.  Gates on different qubits commute, so the gates
-// are applied in groups of up to four on distinct tile positions, each gate
-// after every earlier gate on its own qubit: a thread holds the 2^G
-// amplitudes that a group mixes in registers and applies the group's gates
-// there, one shared-memory sweep and barrier per group instead of per gate
-// (ten gates on qubits 0, 2, ..., 18: three sweeps).  A group takes at most
-// one position below 5 when the tile has 10 or more qubits, which keeps a
-// warp's shared-memory accesses within two-way bank conflicts.  A target
-// outside [0, n) makes every CTA return before it writes (bit 16 of the
-// status word).
+// are applied in groups on distinct tile positions, each gate after every
+// earlier gate on its own qubit: a thread holds the amplitudes that a group
+// mixes in registers, one shared-memory sweep and barrier per group instead of
+// per gate.  A target outside [0, n) makes every CTA return before it writes
+// (bit 16 of the status word).
+//
+// This kernel: states below 12 qubits, one tile, groups of two.  A group takes
+// at most one position below 5 when the tile has 10 or more qubits, which keeps
+// a warp's shared-memory accesses within two-way bank conflicts.
 constexpr int kFusedMax = 12;
 constexpr int kFusedGroup = 2;
 constexpr int kFusedThreads = 512;
@@ -273,6 +273,183 @@ __global__ void __launch_bounds__(kFusedThreads, 2) k_fused1q_dev(float2* __rest
 #pragma unroll 8
     for (uint32_t i = threadIdx.x; i < tsize; i += blockDim.x) s[gbase | dep[0][i & 63] | dep[1][i >> 6]] = tile[i];
     __syncthreads();
+  }
+}
+
+// The same for states of 12 qubits and more: groups of four gates on distinct
+// tile positions, a thread holding the 16 amplitudes that a group mixes; byte
+// addresses built from the columns of the tile's bits; the next tile's 16-byte
+// copies (qubit 0 is in the tile unless twelve other qubits are targets) in
+// flight while one is worked on.
+//
+// Bound by issue: ten gates are 80 FMAs per amplitude, 37 us of FP32 time at 24
+// qubits, as many shared-memory and address instructions, and 41 us of HBM
+// beside them: 115-133 us; 187-202 in sweeps of two gates, which move the tile
+// five times through shared memory.  Three CTAs per SM spill (120 us, and 18.5
+// instead of 14.2 at 20 qubits); registers instead of cp.async cost the same.
+constexpr int kTileThreads = 256;
+
+// The tile's columns: as tile_col, but bit 0 stays with position 0, so that a
+// pair of amplitudes is one 16-byte word (powers of an element of GF(8)).
+__host__ __device__ constexpr uint32_t pair_col(int k) {
+  return k < 4 ? 1u << k : (1u << k) | 2u * (uint32_t)((0x5763421ull >> (4 * ((k - 1) % 7))) & 7);
+}
+__device__ __forceinline__ void copy_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async8(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+
+struct FusedGroup {
+  uint16_t v[4], rem[8];   // byte columns of the register bits and of the thread index
+  int32_t gate[4];         // gate on each register bit, -1 for none
+};
+
+__global__ void __launch_bounds__(kTileThreads, 2)
+    k_fused1q_tiles(float2* __restrict__ s, int n, const float2* __restrict__ gates, const int32_t* __restrict__ targets,
+                    int K, uint32_t* status) {
+  pdl_begin();
+  constexpr int T = kFusedMax;
+  extern __shared__ __align__(16) unsigned char tile_smem[];
+  __shared__ __align__(16) G2 sg[kFusedMax];
+  __shared__ FusedGroup grp[kFusedMax];
+  __shared__ int st[kFusedMax], sq[T];
+  __shared__ uint64_t dep_lo[64], dep_hi[32];   // state index of a pair of amplitudes (tile bits 1-6, 7-11)
+  __shared__ uint16_t map_lo[64], map_hi[32];   // its byte address in the tile
+  __shared__ int s_groups;
+  const int tid = threadIdx.x;
+  if (tid < K) st[tid] = targets[tid];
+  if (tid < 4 * K) sg[tid >> 2].g[tid & 3] = gates[tid];
+  if (tid < 96) {
+    const int first = tid < 64 ? 1 : 7, x = tid < 64 ? tid : tid - 64;
+    uint32_t a = 0;
+    for (int k = 0; k < (tid < 64 ? 6 : 5); ++k)
+      if ((x >> k) & 1) a ^= pair_col(first + k) * 8;
+    if (tid < 64) map_lo[x] = (uint16_t)a; else map_hi[x] = (uint16_t)a;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    uint64_t m = 0;
+    bool ok = true;
+    for (int k = 0; k < K; ++k) {
+      if (st[k] < 0 || st[k] >= n) ok = false;
+      else m |= 1ull << st[k];
+    }
+    int ng = ok ? 0 : -1;
+    if (ok) {
+      for (int q = 0; __popcll(m) < T; ++q) m |= 1ull << q;
+      uint64_t r = m;
+      for (int j = 0; j < T; ++j, r &= r - 1) sq[j] = __ffsll((long long)r) - 1;
+      // a gate joins the group unless it is full or an earlier gate that is
+      // not done has its position
+      for (uint32_t done = 0; done != (1u << K) - 1u; ++ng) {
+        FusedGroup& G = grp[ng];
+        uint32_t seen = 0, bits = 0;
+        int cnt = 0;
+        for (int k = 0; k < K; ++k) {
+          if ((done >> k) & 1) continue;
+          const int p = __popcll(m & ((1ull << st[k]) - 1ull));
+          if (cnt < 4 && !((seen >> p) & 1)) {
+            G.gate[cnt] = k;
+            G.v[cnt++] = (uint16_t)(pair_col(p) * 8);
+            bits |= 1u << p;
+            done |= 1u << k;
+          }
+          seen |= 1u << p;
+        }
+        for (int p = T - 1; cnt < 4; --p)
+          if (!((bits >> p) & 1)) {
+            G.gate[cnt] = -1;
+            G.v[cnt++] = (uint16_t)(pair_col(p) * 8);
+            bits |= 1u << p;
+          }
+        for (int p = 0, j = 0; p < T; ++p)
+          if (!((bits >> p) & 1)) G.rem[j++] = (uint16_t)(pair_col(p) * 8);
+      }
+    } else if (blockIdx.x == 0) {
+      atomicOr(status, 16u);
+    }
+    s_groups = ng;
+  }
+  __syncthreads();
+  const int ngroups = s_groups;
+  if (ngroups < 0) return;
+  const bool pairs = sq[0] == 0;
+  if (tid < 96) {
+    const int first = tid < 64 ? 1 : 7, x = tid < 64 ? tid : tid - 64;
+    uint64_t d = 0;
+    for (int k = 0; k < (tid < 64 ? 6 : 5); ++k)
+      if ((x >> k) & 1) d |= 1ull << sq[first + k];
+    if (tid < 64) dep_lo[x] = d; else dep_hi[x] = d;
+  }
+  __syncthreads();
+  constexpr int kPer = (1 << (T - 1)) / kTileThreads;   // pairs per thread
+  constexpr uint32_t kTile = 8u << T;
+  const uint64_t ntiles = 1ull << (n - T), second = 1ull << sq[0];
+  const uint32_t smem = (uint32_t)__cvta_generic_to_shared(tile_smem);
+  auto first_of = [&](uint64_t tl) {
+    for (int q = 0; q < T; ++q) tl = insert_zero(tl, sq[q]);
+    return tl;
+  };
+  auto fetch = [&](uint64_t tl, uint32_t buf) {
+    const uint64_t gbase = first_of(tl);
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const uint32_t e = tid + kTileThreads * j, A = buf + (map_lo[e & 63] ^ map_hi[e >> 6]);
+      const uint64_t g = gbase | dep_lo[e & 63] | dep_hi[e >> 6];
+      if (pairs) {
+        copy_async16(smem + A, s + g);
+      } else {
+        copy_async8(smem + A, s + g);
+        copy_async8(smem + A + 8, s + (g | second));
+      }
+    }
+  };
+  if (blockIdx.x < ntiles) fetch(blockIdx.x, 0);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  uint32_t buf = 0;
+  for (uint64_t tl = blockIdx.x; tl < ntiles; tl += gridDim.x, buf ^= kTile) {
+    if (tl + gridDim.x < ntiles) fetch(tl + gridDim.x, buf ^ kTile);
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    auto el = [&](uint32_t byte) -> float2& { return *reinterpret_cast<float2*>(tile_smem + byte); };
+    for (int q = 0; q < ngroups; ++q) {
+      const FusedGroup& G = grp[q];
+      uint32_t A = buf;   // a bit above the tile's
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if ((tid >> j) & 1) A ^= G.rem[j];
+      uint32_t at[16];
+      at[0] = A;
+#pragma unroll
+      for (int r = 1; r < 16; ++r) at[r] = at[r & (r - 1)] ^ G.v[31 - __clz(r & -r)];
+      float2 w[16];
+#pragma unroll
+      for (int r = 0; r < 16; ++r) w[r] = el(at[r]);
+      const float4* U = reinterpret_cast<const float4*>(sg);
+      if (G.gate[0] >= 0) gate_on_bit<0>(w, U + 2 * G.gate[0]);
+      if (G.gate[1] >= 0) gate_on_bit<1>(w, U + 2 * G.gate[1]);
+      if (G.gate[2] >= 0) gate_on_bit<2>(w, U + 2 * G.gate[2]);
+      if (G.gate[3] >= 0) gate_on_bit<3>(w, U + 2 * G.gate[3]);
+#pragma unroll
+      for (int r = 0; r < 16; ++r) el(at[r]) = w[r];
+      __syncthreads();
+    }
+    const uint64_t gbase = first_of(tl);
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const uint32_t e = tid + kTileThreads * j, A = map_lo[e & 63] ^ map_hi[e >> 6];
+      const uint64_t g = gbase | dep_lo[e & 63] | dep_hi[e >> 6];
+      const float4 v = *reinterpret_cast<const float4*>(tile_smem + (buf ^ A));
+      if (pairs) {
+        *reinterpret_cast<float4*>(s + g) = v;
+      } else {
+        s[g] = lo2(v);
+        s[g | second] = hi2(v);
+      }
+    }
+    __syncthreads();   // before the buffer is filled again
   }
 }
 
@@ -661,16 +838,23 @@ int qs_apply_gates_fused_dev(qs_handle_t h, void* state, int n, const void* gate
   QS_CHECK_ARG(((uintptr_t)targets_dev & 3u) == 0, "targets must be 4-byte aligned");
   check_dev_ptr(h, targets_dev, "targets");
   const int T = std::min(n, kFusedMax);
-  const size_t smem = sizeof(float2) << T;
   const uint64_t ntiles = 1ull << (n - T);
-  const unsigned grid = (unsigned)std::min<uint64_t>(ntiles, (uint64_t)h->sm_count * 6);
+  // Below 12 qubits the state is one small tile, which groups of two gates and
+  // 512 threads finish sooner; from 12 on k_fused1q_tiles is never behind (ten
+  // gates: 16 qubits 11.8 against 13.2 us, 20 qubits 14.2 / 16.2, 24 qubits 115 /
+  // 187), in one wave of its two CTAs per SM.
+  const bool wide = n >= kFusedMax;
+  const size_t smem = (wide ? 2 : 1) * (sizeof(float2) << T);
+  if (wide) QS_CUDA(cudaFuncSetAttribute(k_fused1q_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const unsigned grid = (unsigned)std::min<uint64_t>(ntiles, (uint64_t)h->sm_count * 2);
   const float2* g = static_cast<const float2*>(gates_dev);
   const int32_t* t = static_cast<const int32_t*>(targets_dev);
   // at most 12 gates per launch, so their distinct targets always fit a tile
   for (int k0 = 0; k0 < n_gates; k0 += kFusedMax) {
     const int K = std::min(kFusedMax, n_gates - k0);
-    k_fused1q_dev<<<grid, kFusedThreads, smem, h->stream>>>((float2*)state, n, g + 4 * k0, t + k0, K, h->dev_status);
-    qs_after_launch(h, "k_fused1q_dev");
+    qs_launch_pdl(h, wide ? k_fused1q_tiles : k_fused1q_dev, dim3(grid), dim3(wide ? kTileThreads : kFusedThreads), smem,
+                  (float2*)state, n, g + 4 * k0, t + k0, K, h->dev_status);
+    qs_after_launch(h, "k_fused1q");
   }
   QS_API_END(h)
 }
