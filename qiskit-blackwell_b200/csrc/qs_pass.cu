@@ -347,6 +347,9 @@ __device__ __forceinline__ void op_dtab(float2 (&v)[1 << R], const DevOp& op, co
       v[j].x = __uint_as_float(__float_as_uint(v[j].x) ^ sb);
       v[j].y = __uint_as_float(__float_as_uint(v[j].y) ^ sb);
     }
+  } else if (op.t0 == 0 && !__any_sync(__activemask(), m)) {  // no sign set in the warp
+#pragma unroll
+    for (int j = 0; j < (1 << R); ++j) v[j] = cmul(v[j], T[j]);
   } else if (op.t0 == 0) {  // table only: the group factor is exactly 1
 #pragma unroll
     for (int j = 0; j < (1 << R); ++j) {
@@ -785,7 +788,10 @@ __device__ __forceinline__ void register_block(float2* tile, const DevBlock& blk
   int pos[R];
   uint32_t pp[R];
 #pragma unroll
-  for (int k = 0; k < R; ++k) { pos[k] = blk.pos[k]; pp[k] = phys(1u << pos[k]); }
+  for (int k = 0; k < R; ++k) { pos[k] = blk.pos[k]; pp[k] = phys(1u << pos[k]) * 8; }
+  auto at = [&](uint32_t byte) -> float2& {
+    return *reinterpret_cast<float2*>(reinterpret_cast<unsigned char*>(tile) + byte);
+  };
   const bool need_g = blk.pos[7] != 0;
   for (uint32_t g = threadIdx.x; g < ngroups; g += blockDim.x) {
     uint32_t base = g;
@@ -799,23 +805,23 @@ __device__ __forceinline__ void register_block(float2* tile, const DevBlock& blk
     float2 v[1 << R];
     // Gray-code walk: consecutive indices differ in one register bit
     {
-      uint32_t a = pb;
+      uint32_t a = pb * 8;   // bytes
 #pragma unroll
       for (int q = 0; q < (1 << R); ++q) {
         const int j = q ^ (q >> 1);
         if (q) a ^= pp[__ffs(q) - 1];
-        v[j] = tile[a];
+        v[j] = at(a);
       }
     }
     if constexpr (TWO == 2) run_ops_u2<R>(v, ops, blk.op_begin, blk.op_end, s_coef);
     else run_ops<R, TWO>(v, ops, blk.op_begin, blk.op_end, s_coef, gidx);
     {
-      uint32_t a = pb;
+      uint32_t a = pb * 8;
 #pragma unroll
       for (int q = 0; q < (1 << R); ++q) {
         const int j = q ^ (q >> 1);
         if (q) a ^= pp[__ffs(q) - 1];
-        tile[a] = v[j];
+        at(a) = v[j];
       }
     }
   }
