@@ -1,11 +1,12 @@
 // qs_batch.cpp — many independent circuits of uneven width in few launches.
 //
 // Every circuit is planned on its own (FP64 fusion + tile passes, in
-// parallel on the host).  Pass p of every circuit that has one is then
-// grouped, by tile size, into one launch of the tile-pass kernel: a circuit
+// parallel on the host).  Pass p of every circuit of one width that has one is
+// then grouped, by tile size, into one launch of the tile-pass kernel: a circuit
 // of <= 14 qubits is a single pass whose tile is the whole state, so it runs
 // start to finish in one CTA's shared memory; wider circuits take several
-// levels.  All device programs live in one buffer and all item tables in
+// levels.  The widths do not depend on one another, so their launches are
+// spread over a few streams and fill each other's last waves.  All device programs live in one buffer and all item tables in
 // another, both built once, so execution issues no host-device copies and can
 // be captured in a CUDA graph.
 //
@@ -16,6 +17,7 @@
 #include <cstdlib>
 #include <algorithm>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <thread>
 #include <tuple>
@@ -32,7 +34,9 @@ struct qs_batch_plan_s {
     uint64_t total_tiles;
     int threads;
     bool tc;  // tensor-core pass (qs_pass_tc.cu)
+    int lane; // launches of one lane run in order, lanes side by side
   };
+  int lanes = 1;
   float* d_mats = nullptr;         // block matrices of the tensor-core launches' passes
   std::vector<Launch> launches;
   qs_batch_info info{};
@@ -179,66 +183,79 @@ qs_batch_plan_s* qs_batch_build_units(qs_context* h, const std::vector<qs_plan_s
     std::vector<std::pair<std::pair<int, int>, size_t>> mat_passes;
     size_t n_mats = 0;
     std::vector<size_t> tc_items;
-    for (int L = 0; L < (queue ? 0 : maxp); ++L) {
-      // key: (T, R, has2); value: items, their plans and the largest coefficient pool
-      struct Group {
-        std::vector<PassItem> items;
-        std::vector<int> plan;
-        int ncoef = 0;
-      };
-      std::map<std::tuple<int, int, int>, Group> groups;
-      for (const BatchUnit& u : units) {
-        const qs_plan_s& p = plans[u.plan];
-        if (L >= (int)p.pass_offsets.size()) continue;
-        const int T = p.pass_T[L];
-        PassItem it{};
-        it.state_off = u.state_off;
-        it.pass = reinterpret_cast<const DevPass*>(static_cast<const char*>(B->d_blob) + boff[u.plan] +
-                                                   p.pass_offsets[L]);
-        it.ntiles = 1ull << (p.n_qubits - T);
-        it.flags = (L == 0 && from_zero) ? PI_FROM_ZERO : 0u;
-        it.noise_seed = u.noise_seed;
-        it.noise_branch = u.noise_branch;
-        auto& g = groups[std::make_tuple(T, p.pass_R[L], p.pass_has2[L])];
-        g.items.push_back(it);
-        g.plan.push_back(u.plan);
-        g.ncoef = std::max(g.ncoef, p.pass_ncoef[L]);
-        bytes += ((L == 0 && from_zero) ? 8.0 : 16.0) * std::ldexp(1.0, p.n_qubits);
-      }
-      // larger tiles first: they are the longest-running CTAs
-      for (auto g = groups.rbegin(); g != groups.rend(); ++g) {
-        qs_batch_plan_s::Launch Lc;
-        Lc.T = std::get<0>(g->first);
-        Lc.R = std::get<1>(g->first);
-        Lc.has2 = std::get<2>(g->first);
-        Lc.ncoef = g->second.ncoef;
-        Lc.item_off = items.size();
-        Lc.n_items = (int)g->second.items.size();
-        Lc.tc = qs_tc_pass(h, Lc.T, Lc.R, Lc.has2);
-        uint64_t tb = 0;
-        for (size_t k = 0; k < g->second.items.size(); ++k) {
-          PassItem it = g->second.items[k];
-          it.tile_begin = tb;
-          tb += it.ntiles;
-          if (Lc.tc) {
-            const int pl = g->second.plan[k];
-            auto key = std::make_pair(pl, L);
-            auto f = mat_first.find(key);
-            if (f == mat_first.end()) {
-              const auto* P = reinterpret_cast<const DevPass*>(plans[pl].blob.data() + plans[pl].pass_offsets[L]);
-              f = mat_first.emplace(key, n_mats).first;
-              mat_passes.push_back({key, n_mats});
-              n_mats += (size_t)P->nblocks;
-            }
-            it.mats = reinterpret_cast<const float*>((uintptr_t)f->second);
-            tc_items.push_back(items.size());
-          }
-          items.push_back(it);
+    // One chain of launches per width, the widest first (they take longest);
+    // each goes to the lane with the least work so far.
+    std::vector<int> widths;
+    for (const BatchUnit& u : units) widths.push_back(plans[u.plan].n_qubits);
+    std::sort(widths.begin(), widths.end(), std::greater<int>());
+    widths.erase(std::unique(widths.begin(), widths.end()), widths.end());
+    std::vector<double> lane_work(std::min<size_t>(widths.size(), kBatchLanes), 0.0);
+    B->lanes = std::max(1, (int)lane_work.size());
+    for (size_t wk = 0; wk < (queue ? 0 : widths.size()); ++wk) {
+      const int lane = (int)(std::min_element(lane_work.begin(), lane_work.end()) - lane_work.begin());
+      for (int L = 0; L < maxp; ++L) {
+        // key: (T, R, has2); value: items, their plans and the largest coefficient pool
+        struct Group {
+          std::vector<PassItem> items;
+          std::vector<int> plan;
+          int ncoef = 0;
+        };
+        std::map<std::tuple<int, int, int>, Group> groups;
+        for (const BatchUnit& u : units) {
+          const qs_plan_s& p = plans[u.plan];
+          if (p.n_qubits != widths[wk] || L >= (int)p.pass_offsets.size()) continue;
+          const int T = p.pass_T[L];
+          PassItem it{};
+          it.state_off = u.state_off;
+          it.pass = reinterpret_cast<const DevPass*>(static_cast<const char*>(B->d_blob) + boff[u.plan] +
+                                                     p.pass_offsets[L]);
+          it.ntiles = 1ull << (p.n_qubits - T);
+          it.flags = (L == 0 && from_zero) ? PI_FROM_ZERO : 0u;
+          it.noise_seed = u.noise_seed;
+          it.noise_branch = u.noise_branch;
+          auto& g = groups[std::make_tuple(T, p.pass_R[L], p.pass_has2[L])];
+          g.items.push_back(it);
+          g.plan.push_back(u.plan);
+          g.ncoef = std::max(g.ncoef, p.pass_ncoef[L]);
+          bytes += ((L == 0 && from_zero) ? 8.0 : 16.0) * std::ldexp(1.0, p.n_qubits);
         }
-        Lc.total_tiles = tb;
-        Lc.threads = threads;
-        B->launches.push_back(Lc);
-        if (Lc.tc) ++B->info.n_tc_launches;
+        // larger tiles first: they are the longest-running CTAs
+        for (auto g = groups.rbegin(); g != groups.rend(); ++g) {
+          qs_batch_plan_s::Launch Lc;
+          Lc.T = std::get<0>(g->first);
+          Lc.R = std::get<1>(g->first);
+          Lc.has2 = std::get<2>(g->first);
+          Lc.ncoef = g->second.ncoef;
+          Lc.item_off = items.size();
+          Lc.n_items = (int)g->second.items.size();
+          Lc.tc = qs_tc_pass(h, Lc.T, Lc.R, Lc.has2);
+          uint64_t tb = 0;
+          for (size_t k = 0; k < g->second.items.size(); ++k) {
+            PassItem it = g->second.items[k];
+            it.tile_begin = tb;
+            tb += it.ntiles;
+            if (Lc.tc) {
+              const int pl = g->second.plan[k];
+              auto key = std::make_pair(pl, L);
+              auto f = mat_first.find(key);
+              if (f == mat_first.end()) {
+                const auto* P = reinterpret_cast<const DevPass*>(plans[pl].blob.data() + plans[pl].pass_offsets[L]);
+                f = mat_first.emplace(key, n_mats).first;
+                mat_passes.push_back({key, n_mats});
+                n_mats += (size_t)P->nblocks;
+              }
+              it.mats = reinterpret_cast<const float*>((uintptr_t)f->second);
+              tc_items.push_back(items.size());
+            }
+            items.push_back(it);
+          }
+          Lc.total_tiles = tb;
+          Lc.threads = threads;
+          Lc.lane = lane;
+          lane_work[lane] += std::ldexp((double)tb, Lc.T);
+          B->launches.push_back(Lc);
+          if (Lc.tc) ++B->info.n_tc_launches;
+        }
       }
     }
     for (const BatchUnit& u : units) flops += plans[u.plan].info.flops;
@@ -319,32 +336,53 @@ static void launch_queue_batch(qs_context* h, qs_batch_plan_s* B, void* states) 
                        B->q_has2, B->q_ncoef, B->d_counters, withhold, limit);
 }
 
-void qs_batch_launch(qs_context* h, qs_batch_plan_s* B, void* states) {
-  B->stream = h->stream;
+// The launches of a plan: lane 0 on the handle's stream, the others on side
+// streams that start after the work queued on it and that it waits for.  A
+// stream that the caller is capturing gets them one after the other.
+static void run_batch(qs_context* h, qs_batch_plan_s* B, void* states, bool own_capture = false) {
   if (B->queue) {
     launch_queue_batch(h, B, states);
     return;
   }
-  for (const auto& L : B->launches) {
-    const PassItem* d = static_cast<const PassItem*>(B->d_items) + L.item_off;
-    if (L.tc) qs_launch_pass_tc(h, states, d, L.n_items, L.total_tiles, L.T);
-    else qs_launch_pass_items(h, states, d, L.n_items, L.total_tiles, L.T, L.R, L.has2, L.ncoef, L.threads);
+  int lanes = B->lanes;
+  cudaStream_t main = h->stream;
+  if (lanes > 1 && main && !own_capture) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    QS_CUDA(cudaStreamIsCapturing(main, &cs));
+    if (cs != cudaStreamCaptureStatusNone) lanes = 1;
   }
+  if (lanes > 1) {
+    qs_side_streams(h);
+    QS_CUDA(cudaEventRecord(h->side_event[0], main));
+    for (int k = 1; k < lanes; ++k) QS_CUDA(cudaStreamWaitEvent(h->side_stream[k], h->side_event[0], 0));
+  }
+  try {
+    for (const auto& L : B->launches) {
+      const PassItem* d = static_cast<const PassItem*>(B->d_items) + L.item_off;
+      h->stream = lanes > 1 && L.lane > 0 ? h->side_stream[L.lane] : main;
+      if (L.tc) qs_launch_pass_tc(h, states, d, L.n_items, L.total_tiles, L.T);
+      else qs_launch_pass_items(h, states, d, L.n_items, L.total_tiles, L.T, L.R, L.has2, L.ncoef, L.threads);
+    }
+  } catch (...) {
+    h->stream = main;
+    for (int k = 1; k < lanes; ++k)   // what was queued comes before anything later on the handle's stream
+      if (cudaEventRecord(h->side_event[k], h->side_stream[k]) == cudaSuccess)
+        cudaStreamWaitEvent(main, h->side_event[k], 0);
+    throw;
+  }
+  h->stream = main;
+  for (int k = 1; k < lanes; ++k) {
+    QS_CUDA(cudaEventRecord(h->side_event[k], h->side_stream[k]));
+    QS_CUDA(cudaStreamWaitEvent(main, h->side_event[k], 0));
+  }
+}
+
+void qs_batch_launch(qs_context* h, qs_batch_plan_s* B, void* states) {
+  B->stream = h->stream;
+  run_batch(h, B, states);
 }
 
 void qs_batch_release(qs_batch_plan_s* B) { free_bplan(B); }
-
-static void run_batch(qs_context* h, qs_batch_plan_s* B, void* states) {
-  if (B->queue) {
-    launch_queue_batch(h, B, states);
-    return;
-  }
-  for (const auto& L : B->launches) {
-    const PassItem* d = static_cast<const PassItem*>(B->d_items) + L.item_off;
-    if (L.tc) qs_launch_pass_tc(h, states, d, L.n_items, L.total_tiles, L.T);
-    else qs_launch_pass_items(h, states, d, L.n_items, L.total_tiles, L.T, L.R, L.has2, L.ncoef, L.threads);
-  }
-}
 
 static bool graphs_enabled() {
   const char* e = std::getenv("QSIM_GRAPHS");
@@ -382,7 +420,7 @@ static void run_batch_graphed(qs_context* h, qs_batch_plan_s* B, void* states) {
     cudaGraph_t g = nullptr;
     h->stream = h->own_stream;
     try {
-      run_batch(h, B, states);
+      run_batch(h, B, states, true);
     } catch (...) {
       h->stream = caller;
       cudaStreamEndCapture(h->own_stream, &g);

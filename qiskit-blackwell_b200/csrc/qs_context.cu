@@ -58,6 +58,13 @@ cudaStream_t qs_upload_stream(qs_context* h) {
   return h->upload_stream;
 }
 
+void qs_side_streams(qs_context* h) {
+  for (int k = 0; k < kBatchLanes; ++k) {
+    if (!h->side_event[k]) QS_CUDA(cudaEventCreateWithFlags(&h->side_event[k], cudaEventDisableTiming));
+    if (k && !h->side_stream[k]) QS_CUDA(cudaStreamCreateWithFlags(&h->side_stream[k], cudaStreamNonBlocking));
+  }
+}
+
 void qs_pool_keep_at_least(int device, uint64_t keep) {
   cudaMemPool_t pool = nullptr;
   if (cudaDeviceGetDefaultMemPool(&pool, device) != cudaSuccess || !pool) return;
@@ -138,6 +145,13 @@ int qs_destroy(qs_handle_t h) {
   if (h->upload_stream) {
     cudaStreamSynchronize(h->upload_stream);
     cudaStreamDestroy(h->upload_stream);
+  }
+  for (int k = 0; k < kBatchLanes; ++k) {
+    if (h->side_stream[k]) {
+      cudaStreamSynchronize(h->side_stream[k]);
+      cudaStreamDestroy(h->side_stream[k]);
+    }
+    if (h->side_event[k]) cudaEventDestroy(h->side_event[k]);
   }
   if (h->scratch) cudaFree(h->scratch);
   if (h->dev_status) cudaFree(h->dev_status);

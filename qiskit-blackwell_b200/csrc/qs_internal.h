@@ -43,6 +43,10 @@ struct qs_context {
   // Host-to-device copies of batch programs, so that building a batch does
   // not wait for the work queued on `stream` (created on first use).
   cudaStream_t upload_stream = nullptr;
+  // Lanes 1.. of a batch (qs_batch.cpp; created on first use), and the events
+  // that tie them to `stream` (0: their start, k: lane k's end).
+  cudaStream_t side_stream[8] = {};
+  cudaEvent_t side_event[8] = {};
   std::string err;
   int tile_bits = 0;    // 0: 13, or the autotuned value for the width
   int block_bits = 0;   // 0: 5 for specialised plans, 4 for the generic kernel
@@ -90,6 +94,9 @@ struct qs_context {
 
 // The handle's upload stream (non-blocking; created on first use).
 cudaStream_t qs_upload_stream(qs_context* h);
+// Creates the handle's side streams and their events.
+constexpr int kBatchLanes = 8;
+void qs_side_streams(qs_context* h);
 
 // Records a launch and checks the launch status.
 void qs_after_launch(qs_context* h, const char* what);
