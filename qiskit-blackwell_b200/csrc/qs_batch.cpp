@@ -165,7 +165,7 @@ qs_batch_plan_s* qs_batch_build_units(qs_context* h, const std::vector<qs_plan_s
           items.push_back(it);
           B->q_maxT = std::max(B->q_maxT, p.pass_T[L]);
           // 2 (dense 4x4 only) survives only if every item has it
-          const int h2 = p.pass_has2[L];
+          const int h2 = p.pass_has2[L] == 3 ? 0 : p.pass_has2[L];   // one general loop for all
           B->q_has2 = items.size() == 1 ? h2 : (B->q_has2 == h2 ? h2 : ((B->q_has2 | h2) ? 1 : 0));
           B->q_ncoef = std::max(B->q_ncoef, p.pass_ncoef[L]);
           bytes += ((L == 0 && from_zero) ? 8.0 : 16.0) * std::ldexp(1.0, p.n_qubits);

@@ -308,7 +308,8 @@ void qs_launch_pass_tc_single(qs_context* h, void* state, const DevPass* d_pass,
 inline bool qs_tc_pass(const qs_context* h, int T, int R, int has2) {
   return qs_tc_enabled(h) && R == 5 && has2 == 2 && (T == 12 || T == 13);
 }
-// has2: the pass (or any item of the launch) holds a two-target op; ncoef:
+// has2: the pass (or any item of the launch) holds a two-target op (2: dense
+// two-qubit ops only, 3: rotations and diagonal tables only); ncoef:
 // the largest coefficient pool (float2) of the launch's passes.
 void qs_launch_pass_single(qs_context* h, void* state, const DevPass* d_pass, int T, int R, uint64_t ntiles,
                            uint32_t flags, int has2, int ncoef);

@@ -1235,7 +1235,11 @@ void encode_pass(int n, const PassPlan& pp, const std::vector<IOp>& ops, std::ve
   R_out = R;
   g_last_devops = (int)dops.size();
   nblocks_out = (int)dblocks.size();
-  has2_out = has2;
+  // 3: rotations and diagonal tables only, for the launch (the record says 0)
+  const bool rot_only = !has2 && std::all_of(dops.begin(), dops.end(), [](const DevOp& d) {
+    return d.kind == DK_KRY || d.kind == DK_DTAB || d.kind == DK_SCALE;
+  });
+  has2_out = rot_only ? 3 : has2;
   ncoef_out = (int)hdr.ncoef;
 }
 
