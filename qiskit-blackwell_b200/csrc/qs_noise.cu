@@ -443,11 +443,13 @@ qs_plan_s whole_state_program(int n, const qs_op* ops, int nops, const std::vect
   std::vector<int> site_of(nops, -1);
   for (size_t k = 0; k < sites.size(); ++k) site_of[sites[k].op] = (int)k;
   std::vector<std::vector<int>> on(n);
-  for (int i = 0; i < nops; ++i)
+  for (int i = 0; i < nops; ++i) {
+    QS_CHECK_ARG(ops[i].nq >= 1 && ops[i].nq <= 8, "op qubit count out of range");
     for (int q = 0; q < ops[i].nq; ++q) {
       qs_check_qubit(ops[i].q[q], n, "op");
       on[ops[i].q[q]].push_back(i);
     }
+  }
   std::vector<size_t> head(n, 0);
   std::vector<char> no_chain(nops, 0);
   auto front = [&](int i, const std::vector<size_t>& at) {

@@ -328,6 +328,8 @@ def lower(circuit: Circuit, strip_measure: bool = True) -> np.ndarray:
                 parts += [_HEAD.pack(OP_MCX, 2, a, b, 0, 0, 0, 0, 0, 0, -1, 0), _ZEROS]
             continue
         kind, param, m = _lower_one(ins)
+        if len(m) > 256:
+            raise ValueError(f"{name}: a matrix of more than 16 entries")
         parts += [_HEAD.pack(kind, nq, *qs, *_NO_QUBITS[8 - nq], param, 0), m]
         if len(m) < 256:
             parts.append(_ZEROS[len(m):])
