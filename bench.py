@@ -919,9 +919,9 @@ def bench_chebyshev(args, dev):
             "config": {"workload": describe("chebyshev", args), "degree": K,
                        "l2": f"3 vectors of {(8 * N) >> 20} MiB (the recurrence re-reads them every degree)"},
             "roofline": {"bound": "hbm", "achieved": ach_pf, "peak": peak, "unit": "GB/s", "frac": ach_pf / peak,
-                         "traffic": None, "peak_source": src, "kernel": "k_chebp_fused (matrix-free, one per degree)",
+                         "traffic": None, "peak_source": src, "kernel": "k_chebp_masks (matrix-free, one per degree)",
                          "algorithmic_bytes_per_launch": algo_pf,
-                         "note": "each amplitude also gathers x_k[i ^ x_t] for every Pauli term (from L2 when the "
+                         "note": "each amplitude also gathers x_k[i ^ x_m] for every X mask of the terms (from L2 when the "
                                  "vector fits there), so the kernel is bound by those gathers, not by its 40 N bytes"},
             "csr_path": {"value": 1.0 / per_csr, "unit": "evolutions/s", "nnz": nnz,
                          "roofline": {"achieved": ach_csr, "frac": ach_csr / peak, "unit": "GB/s",
