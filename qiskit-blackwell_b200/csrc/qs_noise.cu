@@ -437,8 +437,13 @@ qs_plan_s whole_state_program(int n, const qs_op* ops, int nops, const std::vect
   //   * A chain is the next channels, and the permutations and diagonals in front
   //     of them, while they touch at most kGroupQubits qubits: one map in the
   //     kernel (noise_block).
-  //   * Where a dense gate is in front of the next channel, a unitary segment:
-  //     every gate that can run now and that a dense gate among them needs.
+  //   * Where no channel fits a chain (a dense gate is in front of the next one, or
+  //     gates on too many qubits), a unitary segment: every gate that can run now
+  //     and that a dense gate among them needs, and every gate that can run if that
+  //     brings no channel to the front either.  A chain without a channel would
+  //     be decided gate by gate by one warp and sweep the tile for itself: 12
+  //     qubits, 600 controlled phases and one channel per qubit, 1024 trajectories:
+  //     2.16 ms of GPU time in 210 chains, 0.44 in three register blocks and three chains.
   constexpr int kGroupQubits = 4, kGroupOps = 32, kGroupGates = 64;
   std::vector<int> site_of(nops, -1);
   for (size_t k = 0; k < sites.size(); ++k) site_of[sites[k].op] = (int)k;
@@ -487,15 +492,20 @@ qs_plan_s whole_state_program(int n, const qs_op* ops, int nops, const std::vect
     std::sort(got.begin(), got.end());
     return got;
   };
-  auto segment = [&](const std::vector<int>& gates) {
-    std::vector<qs_op> seg;
-    for (int i : gates) {
-      seg.push_back(ops[i]);
-      advance(i, head);
-    }
-    const qs_plan_s p = plan_of(seg);
+  std::vector<int> seg;   // gates of the segment in front of the next chain
+  auto take = [&](const std::vector<int>& gates) {
+    for (int i : gates) advance(i, head);
+    seg.insert(seg.end(), gates.begin(), gates.end());
+  };
+  auto end_segment = [&]() {
+    if (seg.empty()) return;
+    std::sort(seg.begin(), seg.end());
+    std::vector<qs_op> g;
+    for (int i : seg) g.push_back(ops[i]);
+    const qs_plan_s p = plan_of(g);
     m.add_plan(p);
     flops += p.info.flops;
+    seg.clear();
   };
   size_t next = 0;   // channel
   while (next < sites.size()) {
@@ -506,6 +516,7 @@ qs_plan_s whole_state_program(int n, const qs_op* ops, int nops, const std::vect
     size_t ncoef = 0;
     int nch = 0;
     groups.emplace_back();
+    const std::vector<size_t> start(head);
     while (next < sites.size()) {
       int i = sites[next].op;
       if (front(i, head)) {
@@ -546,10 +557,12 @@ qs_plan_s whole_state_program(int n, const qs_op* ops, int nops, const std::vect
       groups.emplace_back();
       advance(i, head);
     }
-    if (nch || !plans.empty()) {
+    if (nch) {
+      end_segment();
       m.add_chain(Q, groups, plans, ncoef);
       continue;
     }
+    head = start;
     const std::vector<int> all = closure();
     std::vector<int> gates;
     uint64_t needed = 0;
@@ -559,11 +572,10 @@ qs_plan_s whole_state_program(int n, const qs_op* ops, int nops, const std::vect
       needed |= qs;
       gates.push_back(all[k]);
     }
-    std::reverse(gates.begin(), gates.end());
-    segment(gates.empty() ? all : gates);
+    take(gates.empty() || !seg.empty() ? all : gates);
   }
-  const std::vector<int> rest = closure();
-  if (!rest.empty()) segment(rest);
+  take(closure());
+  end_segment();
   m.flush(true);
   m.out.info.flops = flops;
   return std::move(m.out);
