@@ -16,6 +16,7 @@
 // (blackwell_backend/chebyshev.py:117-123).
 #include "qs_api.h"
 #include "qs_common.cuh"
+#include "qs_rows.h"
 #include <algorithm>
 #include <vector>
 
@@ -62,14 +63,16 @@ __device__ __forceinline__ float2 row_dot(const int32_t* __restrict__ rp, const 
   // gathers, then the sums (in the row's order).  More of them help the wide
   // rows and only add predicated work to the short ones.
   constexpr int kAhead = V <= 4 ? 2 : 4;
-  for (int32_t j = b + lane; j < e; j += V * kAhead) {
+  for (RowWalk w(b, e, lane); w.more(); w.step(V * kAhead)) {
+    const int32_t* cj = ci + w.at;
+    const float2* vj = val + w.at;
     int32_t col[kAhead];
     float2 v[kAhead], xj[kAhead];
 #pragma unroll
     for (int u = 0; u < kAhead; ++u) {
-      const bool in = j + u * V < e;
-      col[u] = in ? ci[j + u * V] : -1;
-      v[u] = in ? val[j + u * V] : make_float2(0.f, 0.f);
+      const bool in = w.has(u * V);
+      col[u] = in ? cj[u * V] : -1;
+      v[u] = in ? vj[u * V] : make_float2(0.f, 0.f);
     }
 #pragma unroll
     for (int u = 0; u < kAhead; ++u)
