@@ -50,20 +50,15 @@ __device__ __forceinline__ Acc acc_reduce(Acc a) {
   return a;
 }
 
-// Compensated row dot: returns (A x)_r for the row handled by this sub-warp.
-// r < 0 means "no row": the lanes still take part in the shuffles.
-template <int V>
-__device__ __forceinline__ float2 row_dot(const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
-                                          const float2* __restrict__ val, const float2* __restrict__ x, int64_t r,
-                                          int lane) {
-  int32_t b = 0, e = 0;
-  if (r >= 0) { b = rp[r]; e = rp[r + 1]; }
+// Adds a lane's entries of a row, V entries apart, to the sums.  kAhead of them
+// are in flight: their columns and values, then the gathers, then the sums (in
+// the row's order).  More of them help the wide rows and only add predicated
+// work to the short ones.
+template <int V, int kAhead>
+__device__ __forceinline__ float2 row_dot(RowWalk w, const int32_t* __restrict__ ci, const float2* __restrict__ val,
+                                          const float2* __restrict__ x) {
   Acc re{0.f, 0.f}, im{0.f, 0.f};
-  // kAhead entries of a lane in flight: their columns and values, then the
-  // gathers, then the sums (in the row's order).  More of them help the wide
-  // rows and only add predicated work to the short ones.
-  constexpr int kAhead = V <= 4 ? 2 : 4;
-  for (RowWalk w(b, e, lane); w.more(); w.step(V * kAhead)) {
+  for (; w.more(); w.step(V * kAhead)) {
     const int32_t* cj = ci + w.at;
     const float2* vj = val + w.at;
     int32_t col[kAhead];
@@ -91,76 +86,101 @@ __device__ __forceinline__ float2 row_dot(const int32_t* __restrict__ rp, const 
   return make_float2(__fadd_rn(re.s, re.c), __fadd_rn(im.s, im.c));
 }
 
-// Warp-uniform row loop: every warp handles 32/V consecutive rows per
+// store(r, (A x)_r) for every row.  Every warp handles 32/V consecutive rows per
 // iteration, so all 32 lanes always execute the same shuffles.
-#define ROW_LOOP(V, ...)                                                        \
-  const int lane = threadIdx.x & (V - 1);                                        \
-  const int sub = (threadIdx.x & 31) / V;                                        \
-  const int64_t warp = (int64_t)(gtid() >> 5), nwarps = (int64_t)(gstride() >> 5); \
-  constexpr int rpw = 32 / V;                                                    \
-  for (int64_t base = warp * rpw; base < nrows; base += nwarps * rpw) {          \
-    const int64_t r = base + sub;                                                \
-    const bool live = r < nrows;                                                 \
-    __VA_ARGS__                                                                  \
+//
+// Rows of more than 64 V entries wait until the warp's others are done and are
+// then walked by all its lanes, one after the other: V follows the mean row, and a
+// star's centre or an arrowhead's first row in a few lanes would keep its warp
+// long after the rest of the launch (one row of 2^17 entries among rows of 2: 0.96
+// ms, 21 in the one lane of V = 1; among rows of 30: 0.98 / 7.0; 64 V is where
+// the others' wait costs what the wider merge does).  Both walks in one loop cost
+// every matrix registers (48 instead of 32): 11.8 instead of 9.6 ms for the
+// 20-qubit evolution, which this form takes 9.0 against 9.1 without it; rows
+// of 5 take 95 us against 92.
+template <int V, class F>
+__device__ __forceinline__ void for_rows(const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+                                         const float2* __restrict__ val, int64_t nrows, const float2* __restrict__ x,
+                                         F store) {
+  constexpr int kAhead = V <= 4 ? 2 : 4, rpw = 32 / V;
+  const int lane = threadIdx.x & (V - 1);
+  const int sub = (threadIdx.x & 31) / V;
+  const int64_t first = (int64_t)(gtid() >> 5) * rpw, step = (int64_t)(gstride() >> 5) * rpw;
+  bool late = false;
+  for (int64_t base = first; base < nrows; base += step) {
+    const int64_t r = base + sub;
+    const bool live = r < nrows;
+    int32_t b = 0, e = 0;
+    if (live) { b = rp[r]; e = rp[r + 1]; }
+    const bool whole = V < 32 && e - b > 64 * V;
+    late |= whole;
+    const float2 d = row_dot<V, kAhead>(RowWalk(b, whole ? b : e, lane), ci, val, x);
+    if (live && lane == 0 && !whole) store(r, d);
   }
+  if (V == 32 || !__any_sync(0xffffffffu, late)) return;
+  for (int64_t base = first; base < nrows; base += step) {
+    const int64_t r = base + sub;
+    int32_t b = 0, e = 0;
+    if (r < nrows) { b = rp[r]; e = rp[r + 1]; }
+    for (uint32_t rows = __ballot_sync(0xffffffffu, lane == 0 && e - b > 64 * V); rows; rows &= rows - 1) {
+      const int from = __ffs((int)rows) - 1;
+      const float2 d = row_dot<32, kAhead>(
+          RowWalk(__shfl_sync(0xffffffffu, b, from), __shfl_sync(0xffffffffu, e, from), threadIdx.x & 31), ci, val, x);
+      if ((threadIdx.x & 31) == 0) store(base + from / V, d);
+    }
+  }
+}
 
 template <int V>
-__global__ void k_spmv(const int32_t* __restrict__ rp, const int32_t* __restrict__ ci, const float2* __restrict__ val,
-                       int64_t nrows, const float2* __restrict__ x, float2* __restrict__ y, float2 alpha,
-                       float2 beta) {
+__global__ void __launch_bounds__(kThreads, V <= 4 ? 8 : 6)
+    k_spmv(const int32_t* __restrict__ rp, const int32_t* __restrict__ ci, const float2* __restrict__ val,
+           int64_t nrows, const float2* __restrict__ x, float2* __restrict__ y, float2 alpha, float2 beta) {
   pdl_begin();
-  ROW_LOOP(V, {
-    const float2 d = row_dot<V>(rp, ci, val, x, live ? r : -1, lane);
-    if (live && lane == 0) {
-      const float2 yo = y[r];
-      float2 o;
-      o.x = alpha.x * d.x - alpha.y * d.y + (beta.x * yo.x - beta.y * yo.y);
-      o.y = alpha.x * d.y + alpha.y * d.x + (beta.x * yo.y + beta.y * yo.x);
-      y[r] = o;
-    }
-  })
+  for_rows<V>(rp, ci, val, nrows, x, [&](int64_t r, float2 d) {
+    const float2 yo = y[r];
+    float2 o;
+    o.x = alpha.x * d.x - alpha.y * d.y + (beta.x * yo.x - beta.y * yo.y);
+    o.y = alpha.x * d.y + alpha.y * d.x + (beta.x * yo.y + beta.y * yo.x);
+    y[r] = o;
+  });
 }
 
 // Fused Chebyshev degree step.  xprev is overwritten with x_next.
 template <int V>
-__global__ void k_cheb_fused(const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
-                             const float2* __restrict__ val, int64_t nrows, const float2* __restrict__ xk,
-                             float2* __restrict__ xprev, float2* __restrict__ out, float two_scale, float2 c) {
+__global__ void __launch_bounds__(kThreads, V <= 4 ? 8 : 6)
+    k_cheb_fused(const int32_t* __restrict__ rp, const int32_t* __restrict__ ci, const float2* __restrict__ val,
+                 int64_t nrows, const float2* __restrict__ xk, float2* __restrict__ xprev, float2* __restrict__ out,
+                 float two_scale, float2 c) {
   pdl_begin();
-  ROW_LOOP(V, {
-    const float2 d = row_dot<V>(rp, ci, val, xk, live ? r : -1, lane);
-    if (live && lane == 0) {
-      const float2 p = xprev[r];
-      const float2 t = make_float2(fmaf(two_scale, d.x, -p.x), fmaf(two_scale, d.y, -p.y));
-      xprev[r] = t;
-      float2 a = out[r];
-      a.x = fmaf(c.x, t.x, fmaf(-c.y, t.y, a.x));
-      a.y = fmaf(c.x, t.y, fmaf(c.y, t.x, a.y));
-      out[r] = a;
-    }
-  })
+  for_rows<V>(rp, ci, val, nrows, xk, [&](int64_t r, float2 d) {
+    const float2 p = xprev[r];
+    const float2 t = make_float2(fmaf(two_scale, d.x, -p.x), fmaf(two_scale, d.y, -p.y));
+    xprev[r] = t;
+    float2 a = out[r];
+    a.x = fmaf(c.x, t.x, fmaf(-c.y, t.y, a.x));
+    a.y = fmaf(c.x, t.y, fmaf(c.y, t.x, a.y));
+    out[r] = a;
+  });
 }
 
 // x1 = scale * A x0 ; out = c0 * x0 + c1 * x1
 template <int V>
-__global__ void k_cheb_first(const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
-                             const float2* __restrict__ val, int64_t nrows, const float2* __restrict__ x0,
-                             float2* __restrict__ x1, float2* __restrict__ out, float scale, float2 c0, float2 c1) {
+__global__ void __launch_bounds__(kThreads, V <= 4 ? 8 : 6)
+    k_cheb_first(const int32_t* __restrict__ rp, const int32_t* __restrict__ ci, const float2* __restrict__ val,
+                 int64_t nrows, const float2* __restrict__ x0, float2* __restrict__ x1, float2* __restrict__ out,
+                 float scale, float2 c0, float2 c1) {
   pdl_begin();
-  ROW_LOOP(V, {
-    const float2 d = row_dot<V>(rp, ci, val, x0, live ? r : -1, lane);
-    if (live && lane == 0) {
-      const float2 t = make_float2(scale * d.x, scale * d.y);
-      x1[r] = t;
-      const float2 a0 = x0[r];
-      float2 a;
-      a.x = c0.x * a0.x - c0.y * a0.y;
-      a.y = c0.x * a0.y + c0.y * a0.x;
-      a.x = fmaf(c1.x, t.x, fmaf(-c1.y, t.y, a.x));
-      a.y = fmaf(c1.x, t.y, fmaf(c1.y, t.x, a.y));
-      out[r] = a;
-    }
-  })
+  for_rows<V>(rp, ci, val, nrows, x0, [&](int64_t r, float2 d) {
+    const float2 t = make_float2(scale * d.x, scale * d.y);
+    x1[r] = t;
+    const float2 a0 = x0[r];
+    float2 a;
+    a.x = c0.x * a0.x - c0.y * a0.y;
+    a.y = c0.x * a0.y + c0.y * a0.x;
+    a.x = fmaf(c1.x, t.x, fmaf(-c1.y, t.y, a.x));
+    a.y = fmaf(c1.x, t.y, fmaf(c1.y, t.x, a.y));
+    out[r] = a;
+  });
 }
 
 // ---- reference mirrors (chebyshev_sm120.cu:24-91): float4 elementwise ----
