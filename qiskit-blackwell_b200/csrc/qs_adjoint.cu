@@ -1061,8 +1061,8 @@ extern "C" int qs_adjoint_gradient(qs_handle_t h, int n, const qs_op* ops, int n
           d_weights);
       qs_after_launch(h, "k_adj_prepare");
     }
-    QS_CUDA(cudaFuncSetAttribute(k_adj_pass<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_smem[0]));
-    QS_CUDA(cudaFuncSetAttribute(k_adj_pass<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_smem[1]));
+    qs_smem_limit(h, (const void*)k_adj_pass<true>, sizeof(float2) << kAdjTileBits);
+    qs_smem_limit(h, (const void*)k_adj_pass<false>, sizeof(float4) << kAdjTileBits);
   }
 
   // ---- forward

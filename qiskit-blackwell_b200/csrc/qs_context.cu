@@ -58,6 +58,16 @@ cudaStream_t qs_upload_stream(qs_context* h) {
   return h->upload_stream;
 }
 
+void qs_smem_limit(qs_context* h, const void* kernel, size_t most) {
+  static std::mutex mu;
+  static std::set<std::pair<int, const void*>> done;
+  std::lock_guard<std::mutex> lk(mu);
+  const auto key = std::make_pair(h->device, kernel);
+  if (done.count(key)) return;
+  QS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+  done.insert(key);
+}
+
 void qs_side_streams(qs_context* h) {
   for (int k = 0; k < kBatchLanes; ++k) {
     if (!h->side_event[k]) QS_CUDA(cudaEventCreateWithFlags(&h->side_event[k], cudaEventDisableTiming));

@@ -845,7 +845,7 @@ int qs_apply_gates_fused_dev(qs_handle_t h, void* state, int n, const void* gate
   // 187), in one wave of its two CTAs per SM.
   const bool wide = n >= kFusedMax;
   const size_t smem = (wide ? 2 : 1) * (sizeof(float2) << T);
-  if (wide) QS_CUDA(cudaFuncSetAttribute(k_fused1q_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (wide) qs_smem_limit(h, (const void*)k_fused1q_tiles, smem);   // (every call's size is this one)
   const unsigned grid = (unsigned)std::min<uint64_t>(ntiles, (uint64_t)h->sm_count * 2);
   const float2* g = static_cast<const float2*>(gates_dev);
   const int32_t* t = static_cast<const int32_t*>(targets_dev);

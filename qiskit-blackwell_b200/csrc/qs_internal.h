@@ -98,6 +98,12 @@ cudaStream_t qs_upload_stream(qs_context* h);
 constexpr int kBatchLanes = 8;
 void qs_side_streams(qs_context* h);
 
+// Raises a kernel's dynamic shared-memory limit on the handle's device, once.
+// The limit belongs to the function, not to the call: `most` is the largest that
+// any call of the kernel launches with, so that a smaller call on another thread
+// cannot lower it between this thread's check and its launch.
+void qs_smem_limit(qs_context* h, const void* kernel, size_t most);
+
 // Records a launch and checks the launch status.
 void qs_after_launch(qs_context* h, const char* what);
 

@@ -717,6 +717,11 @@ __global__ void __launch_bounds__(kThreads, 3)
 
 struct PauliUpload { const uint32_t* table; PauliRuns runs; size_t bytes; };
 
+// The largest table: 1024 terms of as many masks.  Up to 32 KiB of it, with the
+// static arrays, need no raised limit.
+template <class U>
+constexpr size_t pauli_largest() { return 1024 * (sizeof(PauliMask<U>) + sizeof(PauliTerm<U>)); }
+
 // Builds the table in scratch after `offset` bytes.  `regs`: the index bits a
 // thread holds in registers; `halve`: choose one of the rows i and i ^ x.
 template <class U>
@@ -785,8 +790,7 @@ void pauli_apply(qs_context* h, const float2* in, float2* out, uint64_t vstride,
                  const uint64_t* z, const double* c, int nterms) {
   const PauliUpload T = pauli_upload<U>(h, 0, n, x, z, c, nterms, pauli_regs<M>(), false);
   const uint64_t nthr = (1ull << n) / (2 * M), per = kThreads / S;
-  if (T.bytes > 32 * 1024)   // 48 KiB without the attribute, static arrays included
-    QS_CUDA(cudaFuncSetAttribute(k_pauli_apply<M, S, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T.bytes));
+  if (T.bytes > 32 * 1024) qs_smem_limit(h, (const void*)k_pauli_apply<M, S, U>, pauli_largest<U>());
   qs_launch_pdl(h, k_pauli_apply<M, S, U>, dim3((unsigned)((nthr + per - 1) / per), nb), dim3(kThreads), T.bytes, in, out,
                 vstride, T.table, T.runs, (U)nthr);
   qs_after_launch(h, "k_pauli_apply");
@@ -828,8 +832,7 @@ void pauli_expect(qs_context* h, const float2* psi, int n, const uint64_t* x, co
   const PauliUpload T = pauli_upload<U>(h, 64 + 8 * kMaxBlocks, n, x, z, c, nterms, pauli_regs<M>(), true);
   const uint64_t nthr = (1ull << n) / (2 * M), per = kThreads / S;
   const int nb = (int)std::min<uint64_t>((nthr + per - 1) / per, kPauliBlocks);
-  if (T.bytes > 32 * 1024)   // 48 KiB without the attribute, static arrays included
-    QS_CUDA(cudaFuncSetAttribute(k_pauli_expect<M, S, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T.bytes));
+  if (T.bytes > 32 * 1024) qs_smem_limit(h, (const void*)k_pauli_expect<M, S, U>, pauli_largest<U>());
   qs_launch_pdl(h, k_pauli_expect<M, S, U>, dim3(nb), dim3(kThreads), T.bytes, psi, T.table, T.runs, (U)nthr, red_part(h));
   qs_after_launch(h, "k_pauli_expect");
   qs_launch_pdl(h, k_final, dim3(1), dim3(1024), 0, red_part(h), nb, red_out(h), 0);
