@@ -93,11 +93,12 @@ __device__ __forceinline__ float2 row_dot(RowWalk w, const int32_t* __restrict__
 // then walked by all its lanes, one after the other: V follows the mean row, and a
 // star's centre or an arrowhead's first row in a few lanes would keep its warp
 // long after the rest of the launch (one row of 2^17 entries among rows of 2: 0.96
-// ms, 21 in the one lane of V = 1; among rows of 30: 0.98 / 7.0; 64 V is where
-// the others' wait costs what the wider merge does).  Both walks in one loop cost
-// every matrix registers (48 instead of 32): 11.8 instead of 9.6 ms for the
-// 20-qubit evolution, which this form takes 9.0 against 9.1 without it; rows
-// of 5 take 95 us against 92.
+// ms, 21 in the one lane of V = 1; among rows of 30: 0.98 / 7.0).  64 V leaves rows of
+// twice the mean in their own lanes; Pareto rows (mean 5, exponent 1.3) take 204 /
+// 218 / 243 us for 32 V / 64 V / 128 V, rows of one length the same.  Both walks in
+// one loop cost every matrix registers (48 instead of 32): 11.8 instead of 9.6 ms
+// for the 20-qubit evolution, which this form takes 9.0 against 9.1 without it;
+// rows of 5 take 95 us against 92.
 template <int V, class F>
 __device__ __forceinline__ void for_rows(const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
                                          const float2* __restrict__ val, int64_t nrows, const float2* __restrict__ x,
@@ -117,16 +118,18 @@ __device__ __forceinline__ void for_rows(const int32_t* __restrict__ rp, const i
     const float2 d = row_dot<V, kAhead>(RowWalk(b, whole ? b : e, lane), ci, val, x);
     if (live && lane == 0 && !whole) store(r, d);
   }
-  if (V == 32 || !__any_sync(0xffffffffu, late)) return;
-  for (int64_t base = first; base < nrows; base += step) {
-    const int64_t r = base + sub;
-    int32_t b = 0, e = 0;
-    if (r < nrows) { b = rp[r]; e = rp[r + 1]; }
-    for (uint32_t rows = __ballot_sync(0xffffffffu, lane == 0 && e - b > 64 * V); rows; rows &= rows - 1) {
-      const int from = __ffs((int)rows) - 1;
-      const float2 d = row_dot<32, kAhead>(
-          RowWalk(__shfl_sync(0xffffffffu, b, from), __shfl_sync(0xffffffffu, e, from), threadIdx.x & 31), ci, val, x);
-      if ((threadIdx.x & 31) == 0) store(base + from / V, d);
+  if constexpr (V < 32) {
+    if (!__any_sync(0xffffffffu, late)) return;
+    for (int64_t base = first; base < nrows; base += step) {
+      const int64_t r = base + sub;
+      int32_t b = 0, e = 0;
+      if (r < nrows) { b = rp[r]; e = rp[r + 1]; }
+      for (uint32_t rows = __ballot_sync(0xffffffffu, lane == 0 && e - b > 64 * V); rows; rows &= rows - 1) {
+        const int from = __ffs((int)rows) - 1;
+        const RowWalk w(__shfl_sync(0xffffffffu, b, from), __shfl_sync(0xffffffffu, e, from), threadIdx.x & 31);
+        const float2 d = row_dot<32, kAhead>(w, ci, val, x);
+        if ((threadIdx.x & 31) == 0) store(base + from / V, d);
+      }
     }
   }
 }
