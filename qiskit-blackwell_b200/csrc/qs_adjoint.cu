@@ -817,6 +817,8 @@ struct AdjPlan {
         pending[pos[o.q[0]]].push_back(i);
         continue;
       }
+      // an X controlled by its own target never acts
+      if (o.kind == QS_OP_MCX && std::find(o.q, o.q + o.nq - 1, o.q[o.nq - 1]) != o.q + o.nq - 1) continue;
       uint32_t need = 0;
       for (int q = 0; q < o.nq; ++q)
         if (pos[o.q[q]] >= 0) need |= 1u << pos[o.q[q]];
@@ -916,7 +918,8 @@ struct AdjPlan {
           if (done[k] || (targ[k] & ~S) || !ready(k)) continue;
           done[k] = 1;
           --remaining;
-          for (uint64_t t = touch[k]; t; t &= t - 1) ++head[__builtin_ctzll(t)];
+          const qs_op& o = ops[order[k]];   // a qubit may be listed twice
+          for (int q = 0; q < o.nq; ++q) ++head[o.q[q]];
           cur.push_back(k);
           progress = true;
         }
