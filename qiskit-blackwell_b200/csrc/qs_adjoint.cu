@@ -11,8 +11,8 @@
 // and lambda, cross HBM once per pass instead of once per gate, and CTAs apply
 // the gates of a pass to a tile in shared memory.  The FP64 partial sums of
 // <lambda|P|psi> are reduced in a fixed order (deterministic).
-// QSIM_ADJ_PASSES=0, or very many partials, selects the older sweep (a
-// batch-planned forward, then one launch per gate; kept for comparison).
+// QSIM_ADJ_PASSES=0 selects the older sweep (a batch-planned forward, then one
+// launch per gate; kept for comparison).
 // There is no reference counterpart (ROADMAP.md:173-175 lists adjoint
 // differentiation as future work).
 #include "qs_api.h"
@@ -221,7 +221,7 @@ struct PassArg {
   int32_t S[kAdjTileBits];  // tile positions (global qubits), ascending
   int32_t T, bits;    // tile bits, and those of them that exist (n < T)
   int32_t gb, ge;     // steps of the pass
-  int32_t nslots;     // sums of the whole sweep
+  int32_t slot0, nslots;  // first sum of the pass's part of the sweep, and how many it has
   int32_t from_zero;  // forward: the tile starts as |0..0> instead of being loaded
 };
 
@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(kThreads, FWD ? 3 : 2)
       double t = 0.0;
 #pragma unroll
       for (int w = 0; w < kThreads / 32; ++w) t += red[cur][w][tid];
-      partial[((uint64_t)b * P.nslots + G.slot[tid / 3] + tid % 3) * ntiles + tile] = t;
+      partial[((uint64_t)b * P.nslots + G.slot[tid / 3] - P.slot0 + tid % 3) * ntiles + tile] = t;
     }
     __syncwarp();   // the step is read above and its buffer refilled by this warp
   }
@@ -617,13 +617,13 @@ __global__ void k_adj_prepare(const AdjRun* __restrict__ runs, int nruns, const 
 // A parameter gate: the first of its run's sums, and which weights it has.
 struct AdjRef { int32_t slot, w; };
 
-// grads[b][p] = sum over the gates with parameter p of its axis . (sums over
-// the tiles), one warp per (p, b), in a fixed order.
+// grads[b][p] += sum over a part's gates with parameter p of its axis . (sums
+// over the tiles), one warp per (p, b), in a fixed order.
 __global__ void k_adj_grads(const double* __restrict__ partial, int nslots, uint64_t ntiles,
                             const int32_t* __restrict__ first, const AdjRef* __restrict__ refs,
                             const double* __restrict__ weights, int nb, double* __restrict__ grads, int nparams) {
   const int p = (int)(gtid() >> 5), lane = threadIdx.x & 31, b = blockIdx.y;
-  if (p >= nparams) return;
+  if (p >= nparams || first[p] == first[p + 1]) return;
   double total = 0.0;
   for (int k = first[p]; k < first[p + 1]; ++k) {
     const AdjRef R = refs[k];
@@ -637,7 +637,7 @@ __global__ void k_adj_grads(const double* __restrict__ partial, int nslots, uint
     const double* w = weights + ((uint64_t)R.w * nb + b) * 3;
     total += w[0] * warp_sum(x) + w[1] * warp_sum(y) + w[2] * warp_sum(z);
   }
-  if (lane == 0) grads[(uint64_t)b * nparams + p] = total;
+  if (lane == 0) grads[(uint64_t)b * nparams + p] += total;
 }
 
 SortedQ sortedq(std::vector<int> q) {
@@ -673,6 +673,13 @@ bool adj_passes_enabled() {
   return on;
 }
 
+// Bytes of partial sums held at a time.  28 qubits, 40 layers of RY and CX chains
+// (1120 runs of three sums): 801 ms in two parts, 5336 in one launch per gate.
+constexpr size_t kAdjPartials = 3ull << 29;
+
+// Reverse passes [pass0, pass1) and their sums.
+struct AdjPart { size_t pass0, pass1; int32_t slot0, nslots; };
+
 bool is_1q_kind(int k) {
   return k == QS_OP_RX || k == QS_OP_RY || k == QS_OP_RZ || k == QS_OP_U1 || k == QS_OP_DIAG1 || k == QS_OP_Y;
 }
@@ -690,6 +697,7 @@ struct AdjPlan {
   std::vector<AdjRef> refs;
   std::vector<int32_t> ref_param;
   int nslots = 0;
+  size_t max_params = ~size_t(0);  // parameter gates of a reverse pass
 
   // state of the pass that is being cut into steps
   int pos[64];
@@ -809,6 +817,7 @@ struct AdjPlan {
     for (int j = 0; j < T; ++j) col[j] = tile_col(j);
     cst = 0;
     out.clear();
+    P.slot0 = nslots;
     P.gb = (int)steps.size();
     for (size_t at = 0; at < cur.size(); ++at) {
       const int i = cur[at];
@@ -862,6 +871,7 @@ struct AdjPlan {
     if (count) block(which, count);
     steps.push_back(step(AG_STORE));
     P.ge = (int)steps.size();
+    P.nslots = nslots - P.slot0;
     passes.push_back(P);
   }
 
@@ -899,7 +909,9 @@ struct AdjPlan {
     const uint64_t lows = (1ull << (bits == n ? n : L)) - 1;
     uint64_t S = lows;
     std::vector<int> cur;
+    size_t params = 0;   // parameter gates in cur
     auto close = [&]() {
+      params = 0;
       for (int q = 0; __builtin_popcountll(S) < bits && q < n; ++q) S |= 1ull << q;  // fill the tile
       // back in the order of the sweep (it respects every dependency): taken as
       // the tile grew, a layer's gates would be scattered over many blocks
@@ -922,6 +934,7 @@ struct AdjPlan {
           for (int q = 0; q < o.nq; ++q) ++head[o.q[q]];
           cur.push_back(k);
           progress = true;
+          if (rev && o.param >= 0 && ++params >= max_params) close();
         }
         while (first < m && done[first]) ++first;
       }
@@ -973,18 +986,34 @@ extern "C" int qs_adjoint_gradient(qs_handle_t h, int n, const qs_op* ops, int n
   const uint64_t ntiles = 1ull << std::max(0, n - T);
   AdjPlan plan{n, T, std::min(n, kAdjLowQubits), ops};
   std::vector<PassArg> fpasses, rpasses;
-  bool use_passes = adj_passes_enabled();
+  std::vector<AdjPart> parts;
+  size_t part_slots = 1;
+  const bool use_passes = adj_passes_enabled();
   if (use_passes) {
     std::vector<int> order(nops);
     for (int i = 0; i < nops; ++i) order[i] = i;
     plan.sweep(order, false, fpasses);
     std::reverse(order.begin(), order.end());
+    // At most three sums per parameter gate, each an FP64 partial per vector and
+    // tile.  The reverse passes are run in parts of at most kAdjPartials of them,
+    // whose gradients are added up before the next part writes its own.
+    plan.max_params = std::max<size_t>(1, kAdjPartials / (3 * sizeof(double) * nb * ntiles));
     plan.sweep(order, true, rpasses);
     fpasses[0].from_zero = 1;
-    for (auto& P : rpasses) P.nslots = plan.nslots;
-    // one FP64 partial per (vector, sum, tile); past 1.5 GiB of them the
-    // per-gate sweep (partials per block) is used
-    use_passes = (double)nb * std::max(plan.nslots, 1) * (double)ntiles * sizeof(double) <= 1.5 * (double)(1ull << 30);
+    const size_t most = std::max<size_t>(3, kAdjPartials / (sizeof(double) * nb * ntiles));
+    for (size_t k = 0; k < rpasses.size(); ++k) {
+      const PassArg& P = rpasses[k];
+      if (parts.empty() || (size_t)(parts.back().nslots + P.nslots) > most) parts.push_back({k, k, P.slot0, 0});
+      parts.back().pass1 = k + 1;
+      parts.back().nslots += P.nslots;
+    }
+    for (const AdjPart& A : parts) {
+      part_slots = std::max(part_slots, (size_t)A.nslots);
+      for (size_t k = A.pass0; k < A.pass1; ++k) {
+        rpasses[k].slot0 = A.slot0;
+        rpasses[k].nslots = A.nslots;
+      }
+    }
   }
 
   // device buffer: grads [nb][nparams] | energies [nb] | partial [nb][256] | U^dag table of the per-gate sweep
@@ -1022,13 +1051,24 @@ extern "C" int qs_adjoint_gradient(qs_handle_t h, int n, const qs_op* ops, int n
   double *d_weights = nullptr, *d_parts = nullptr;
   const size_t pass_smem[2] = {sizeof(float2) << T, sizeof(float4) << T};
   if (use_passes) {
-    // the gates of each parameter, in the order of the sweep
-    std::vector<int32_t> pfirst(nparams + 1, 0);
-    for (int32_t p : plan.ref_param) ++pfirst[p + 1];
-    for (int p = 0; p < nparams; ++p) pfirst[p + 1] += pfirst[p];
+    // the gates of each parameter, part by part, in the order of the sweep
+    const size_t row = (size_t)nparams + 1;
+    std::vector<int32_t> pfirst(parts.size() * row, 0);
     std::vector<AdjRef> refs(plan.refs.size());
-    std::vector<int32_t> fill(pfirst);
-    for (size_t k = 0; k < refs.size(); ++k) refs[fill[plan.ref_param[k]]++] = plan.refs[k];
+    size_t r = 0;
+    for (size_t k = 0; k < parts.size(); ++k) {
+      int32_t* f = pfirst.data() + k * row;
+      const size_t r0 = r;
+      for (; r < refs.size() && plan.refs[r].slot < parts[k].slot0 + parts[k].nslots; ++r) ++f[plan.ref_param[r] + 1];
+      f[0] = (int32_t)r0;
+      for (int p = 0; p < nparams; ++p) f[p + 1] += f[p];
+      std::vector<int32_t> fill(f, f + nparams);
+      for (size_t q = r0; q < r; ++q) {
+        AdjRef R = plan.refs[q];
+        R.slot -= parts[k].slot0;
+        refs[fill[plan.ref_param[q]]++] = R;
+      }
+    }
     std::vector<char> host;
     size_t off[8];
     auto put = [&](int k, const void* d, size_t size) {
@@ -1044,9 +1084,9 @@ extern "C" int qs_adjoint_gradient(qs_handle_t h, int n, const qs_op* ops, int n
     put(5, plan.run_ops.data(), plan.run_ops.size() * sizeof(AdjOp));
     put(6, plan.consts.data(), plan.consts.size() * sizeof(double));
     put(7, params, sizeof(double) * (size_t)nb * nparams);
-    const size_t parts = (size_t)nb * std::max(plan.nslots, 1) * ntiles, nmats = plan.steps.size() * 4 * nb;
+    const size_t npartials = (size_t)nb * part_slots * ntiles, nmats = plan.steps.size() * 4 * nb;
     QS_CUDA(cudaMallocAsync(&pbuf, host.size() + sizeof(Mat2) * nmats +
-                            sizeof(double) * (parts + 3 * (size_t)nb * refs.size()), h->stream));
+                            sizeof(double) * (npartials + 3 * (size_t)nb * refs.size()), h->stream));
     char* pc = static_cast<char*>(pbuf);
     d_steps = reinterpret_cast<AdjStep*>(pc + off[0]);
     d_mats = reinterpret_cast<float4*>(pc + host.size());
@@ -1054,7 +1094,7 @@ extern "C" int qs_adjoint_gradient(qs_handle_t h, int n, const qs_op* ops, int n
     d_refs = reinterpret_cast<AdjRef*>(pc + off[3]);
     d_first = reinterpret_cast<int32_t*>(pc + off[4]);
     d_parts = reinterpret_cast<double*>(pc + host.size() + sizeof(Mat2) * nmats);
-    d_weights = d_parts + parts;
+    d_weights = d_parts + npartials;
     QS_CUDA(cudaMemcpyAsync(pc, host.data(), host.size(), cudaMemcpyHostToDevice, h->stream));
     const int nruns = (int)plan.runs.size();
     if (nruns) {
@@ -1107,15 +1147,17 @@ extern "C" int qs_adjoint_gradient(qs_handle_t h, int n, const qs_op* ops, int n
 
   // ---- reverse sweep
   if (use_passes) {
-    for (const PassArg& P : rpasses) {
-      k_adj_pass<false><<<dim3((unsigned)ntiles, nb), kThreads, pass_smem[1], h->stream>>>(
-          (float2*)work, vstride, P, d_steps, d_mats, nb, d_u2, d_parts);
-      qs_after_launch(h, "k_adj_pass");
-    }
-    if (nparams > 0) {
-      k_adj_grads<<<dim3((unsigned)((nparams + 3) / 4), nb), 128, 0, h->stream>>>(
-          d_parts, plan.nslots, ntiles, d_first, d_refs, d_weights, nb, d_grads, nparams);
-      qs_after_launch(h, "k_adj_grads");
+    for (size_t k = 0; k < parts.size(); ++k) {
+      for (size_t q = parts[k].pass0; q < parts[k].pass1; ++q) {
+        k_adj_pass<false><<<dim3((unsigned)ntiles, nb), kThreads, pass_smem[1], h->stream>>>(
+            (float2*)work, vstride, rpasses[q], d_steps, d_mats, nb, d_u2, d_parts);
+        qs_after_launch(h, "k_adj_pass");
+      }
+      if (parts[k].nslots > 0) {
+        k_adj_grads<<<dim3((unsigned)((nparams + 3) / 4), nb), 128, 0, h->stream>>>(
+            d_parts, parts[k].nslots, ntiles, d_first + k * (nparams + 1), d_refs, d_weights, nb, d_grads, nparams);
+        qs_after_launch(h, "k_adj_grads");
+      }
     }
   } else
   for (int i = nops - 1; i >= 0; --i) {
