@@ -199,6 +199,7 @@ qs_batch_plan_s* qs_batch_build_units(qs_context* h, const std::vector<qs_plan_s
           std::vector<PassItem> items;
           std::vector<int> plan;
           int ncoef = 0;
+          uint64_t tiles = 0;
         };
         std::map<std::tuple<int, int, int>, Group> groups;
         for (const BatchUnit& u : units) {
@@ -216,8 +217,30 @@ qs_batch_plan_s* qs_batch_build_units(qs_context* h, const std::vector<qs_plan_s
           auto& g = groups[std::make_tuple(T, p.pass_R[L], p.pass_has2[L])];
           g.items.push_back(it);
           g.plan.push_back(u.plan);
+          g.tiles += it.ntiles;
           g.ncoef = std::max(g.ncoef, p.pass_ncoef[L]);
           bytes += ((L == 0 && from_zero) ? 8.0 : 16.0) * std::ldexp(1.0, p.n_qubits);
+        }
+        // Passes of rotations and tables (3) have an op loop of their own; the general
+        // loop (0) runs them too, with the same bits but up to a tenth slower.  A level
+        // that has both is one launch of the general loop, unless each of the two
+        // would fill the GPU for four waves of two CTAs per SM.  Half of the circuits
+        // with a Toffoli in the pass, one launch against two: 8 of 12 qubits 127 us /
+        // 234, 16 of 17 qubits 556 / 733, 16 of 20 qubits (3.5 waves each) 3.42 ms /
+        // 3.53, 4096 of 12 qubits (7 waves) 767 us / 767, 8 of 24 qubits (27 waves)
+        // 30.7 ms / 29.3.
+        for (auto g = groups.begin(); g != groups.end();) {
+          auto general = groups.find(std::make_tuple(std::get<0>(g->first), std::get<1>(g->first), 0));
+          if (std::get<2>(g->first) != 3 || general == groups.end() ||
+              std::min(g->second.tiles, general->second.tiles) >= (uint64_t)h->sm_count * 8) {
+            ++g;
+            continue;
+          }
+          Group& to = general->second;
+          to.items.insert(to.items.end(), g->second.items.begin(), g->second.items.end());
+          to.plan.insert(to.plan.end(), g->second.plan.begin(), g->second.plan.end());
+          to.ncoef = std::max(to.ncoef, g->second.ncoef);
+          g = groups.erase(g);
         }
         // larger tiles first: they are the longest-running CTAs
         for (auto g = groups.rbegin(); g != groups.rend(); ++g) {
