@@ -191,6 +191,7 @@ qs_batch_plan_s* qs_batch_build_units(qs_context* h, const std::vector<qs_plan_s
     widths.erase(std::unique(widths.begin(), widths.end()), widths.end());
     std::vector<double> lane_work(std::min<size_t>(widths.size(), kBatchLanes), 0.0);
     B->lanes = std::max(1, (int)lane_work.size());
+    if (B->lanes > 1) qs_side_streams(h);   // before any capture
     for (size_t wk = 0; wk < (queue ? 0 : widths.size()); ++wk) {
       const int lane = (int)(std::min_element(lane_work.begin(), lane_work.end()) - lane_work.begin());
       for (int L = 0; L < maxp; ++L) {
@@ -360,20 +361,16 @@ static void launch_queue_batch(qs_context* h, qs_batch_plan_s* B, void* states) 
 }
 
 // The launches of a plan: lane 0 on the handle's stream, the others on side
-// streams that start after the work queued on it and that it waits for.  A
-// stream that the caller is capturing gets them one after the other.
-static void run_batch(qs_context* h, qs_batch_plan_s* B, void* states, bool own_capture = false) {
+// streams that start after the work queued on it and that it waits for.  In a
+// capture, the plan's own or the caller's, the two events make the lanes branches
+// of the graph (widths 15 to 20, four of each: 1437 us replayed; 3169 in a row).
+static void run_batch(qs_context* h, qs_batch_plan_s* B, void* states) {
   if (B->queue) {
     launch_queue_batch(h, B, states);
     return;
   }
-  int lanes = B->lanes;
+  const int lanes = B->lanes;
   cudaStream_t main = h->stream;
-  if (lanes > 1 && main && !own_capture) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    QS_CUDA(cudaStreamIsCapturing(main, &cs));
-    if (cs != cudaStreamCaptureStatusNone) lanes = 1;
-  }
   if (lanes > 1) {
     qs_side_streams(h);
     QS_CUDA(cudaEventRecord(h->side_event[0], main));
@@ -443,7 +440,7 @@ static void run_batch_graphed(qs_context* h, qs_batch_plan_s* B, void* states) {
     cudaGraph_t g = nullptr;
     h->stream = h->own_stream;
     try {
-      run_batch(h, B, states, true);
+      run_batch(h, B, states);
     } catch (...) {
       h->stream = caller;
       cudaStreamEndCapture(h->own_stream, &g);
