@@ -106,9 +106,11 @@ __global__ void k_1q_tn(float2* __restrict__ s, uint64_t nitems, int t, G2 G0, c
 // per gate.  A target outside [0, n) makes every CTA return before it writes
 // (bit 16 of the status word).
 //
-// This kernel: states below 12 qubits, one tile, groups of two.  A group takes
-// at most one position below 5 when the tile has 10 or more qubits, which keeps
-// a warp's shared-memory accesses within two-way bank conflicts.
+// This kernel: states below 12 qubits, one CTA whose tile is the state, groups of
+// two.  A group takes at most one position below 5 from 10 qubits on, which keeps a
+// warp's shared-memory accesses within two-way bank conflicts.  Bound by latency (one
+// round trip, thread 0's grouping, a sweep and a barrier per group): ten gates on 10
+// qubits 5.3 us of GPU time, 7.0 with the tables of a kernel for wider states.
 constexpr int kFusedMax = 12;
 constexpr int kFusedGroup = 2;
 constexpr int kFusedThreads = 512;
@@ -118,12 +120,12 @@ constexpr int kFusedThreads = 512;
 // amplitudes; srt = the group's positions ascending.
 template <int G>
 __device__ __forceinline__ void fused_group_sweep(float2* __restrict__ tile, uint32_t tsize, const int* gidx,
-                                                  const int* srt_s, const G2* sg, const int* spos) {
+                                                  const int* srt_s, const G2* sg, const int* targets) {
   int pos[G], srt[G];
   G2 M[G];
 #pragma unroll
   for (int b = 0; b < G; ++b) {
-    pos[b] = spos[gidx[b]];
+    pos[b] = targets[gidx[b]];
     M[b] = sg[gidx[b]];
     srt[b] = srt_s[b];
   }
@@ -165,66 +167,52 @@ __global__ void __launch_bounds__(kFusedThreads, 2) k_fused1q_dev(float2* __rest
   pdl_begin();
   extern __shared__ float2 tile[];
   __shared__ G2 sg[kFusedMax];
-  __shared__ int st[kFusedMax];     // targets
-  __shared__ int spos[kFusedMax];   // tile position of gate k's target
-  __shared__ int sq[kFusedMax];     // tile qubits, ascending
-  __shared__ uint64_t dep[2][64];   // tile index bits -> state index bits (6 + 6)
+  __shared__ int st[kFusedMax];                 // targets, which are the tile positions
   __shared__ int gidx[kFusedMax][kFusedGroup];  // groups: gate indices, application order
   __shared__ int gsrt[kFusedMax][kFusedGroup];  // groups: tile positions ascending
   __shared__ int gsize[kFusedMax];
-  __shared__ int s_ngroups;
-  __shared__ int s_ok;
-  const int T = n < kFusedMax ? n : kFusedMax;
-  // one round trip for the gates' matrices and targets, then thread 0 picks
-  // the tile qubits from shared memory
+  __shared__ int s_ngroups;                     // -1: a target is out of range
+  // one round trip for the gates' matrices, the targets and the state; then
+  // thread 0 groups the gates from shared memory
   if ((int)threadIdx.x < K) st[threadIdx.x] = targets[threadIdx.x];
   if ((int)threadIdx.x < 4 * K) sg[threadIdx.x >> 2].g[threadIdx.x & 3] = gates[threadIdx.x];
+  const uint32_t tsize = 1u << n;
+#pragma unroll 4
+  for (uint32_t i = threadIdx.x; i < tsize; i += kFusedThreads) tile[i] = s[i];
   __syncthreads();
   if (threadIdx.x == 0) {
-    // thread 0 alone, while the CTA waits at the barrier: the targets and
-    // positions live in registers (loops unrolled over kFusedMax), so the
-    // setup costs no shared-memory round trips
+    // thread 0 alone, while the CTA waits at the barrier: the targets live in
+    // registers (loops unrolled over kFusedMax), so the setup costs no
+    // shared-memory round trips
     int tg[kFusedMax];
-    uint64_t m = 0;
-    int ok = 1;
+    bool ok = true;
 #pragma unroll
     for (int k = 0; k < kFusedMax; ++k) {
       tg[k] = k < K ? st[k] : 0;
-      if (k < K) {
-        if (tg[k] < 0 || tg[k] >= n) ok = 0; else m |= 1ull << tg[k];
-      }
+      if (tg[k] < 0 || tg[k] >= n) ok = false;
     }
-    for (int q = 0; q < n && __popcll(m) < T; ++q) m |= 1ull << q;
-    {
-      uint64_t r = m;
-      for (int j = 0; r != 0; ++j, r &= r - 1) sq[j] = __ffsll((long long)r) - 1;
-    }
+    int ng = ok ? 0 : -1;
     if (ok) {
-      int sp[kFusedMax];
       uint32_t same[kFusedMax];  // earlier gates on the same position
 #pragma unroll
       for (int k = 0; k < kFusedMax; ++k) {
-        sp[k] = __popcll(m & ((1ull << tg[k]) - 1ull));
-        spos[k] = sp[k];
         same[k] = 0;
 #pragma unroll
         for (int k2 = 0; k2 < k; ++k2)
-          if (sp[k2] == sp[k]) same[k] |= 1u << k2;
+          if (tg[k2] == tg[k]) same[k] |= 1u << k2;
       }
       // groups: scan the unscheduled gates in order and take gate k unless
       // an earlier unscheduled gate (in this group or later) has its
       // position, the group is full, or it would be a second low position
-      const int lowlim = T >= 10 ? 5 : 0;
+      const int lowlim = n >= 10 ? 5 : 0;
       const uint32_t all = (1u << K) - 1u;
-      uint32_t done = 0;
-      int ng = 0;
-      while (done != all) {
+      for (uint32_t done = 0; done != all; ++ng) {
         int cnt = 0;
         uint32_t used = 0, pick = 0;
         bool low = false;
 #pragma unroll
         for (int k = 0; k < kFusedMax; ++k) {
-          const int p = sp[k];
+          const int p = tg[k];
           if (k < K && cnt < kFusedGroup && !((done >> k) & 1u) && !(same[k] & ~done) && !(p < lowlim && low)) {
             gidx[ng][cnt++] = k;
             used |= 1u << p;
@@ -235,45 +223,24 @@ __global__ void __launch_bounds__(kFusedThreads, 2) k_fused1q_dev(float2* __rest
         done |= pick;
         uint32_t r = used;
         for (int j = 0; r != 0; ++j, r &= r - 1) gsrt[ng][j] = __ffs((int)r) - 1;
-        gsize[ng++] = cnt;
+        gsize[ng] = cnt;
       }
-      s_ngroups = ng;
-    } else if (blockIdx.x == 0) {
+    } else {
       atomicOr(status, 16u);
     }
-    s_ok = ok;
+    s_ngroups = ng;
   }
   __syncthreads();
-  if (!s_ok) return;
-  for (int e = threadIdx.x; e < 128; e += blockDim.x) {
-    const int part = e >> 6, x = e & 63;
-    uint64_t d = 0;
-    for (int b = 0; b < 6; ++b) {
-      const int kk = 6 * part + b;
-      if (kk < T && ((x >> b) & 1)) d |= 1ull << sq[kk];
+  if (s_ngroups < 0) return;
+  for (int g = 0; g < s_ngroups; ++g) {
+    switch (gsize[g]) {
+      case 1: fused_group_sweep<1>(tile, tsize, gidx[g], gsrt[g], sg, st); break;
+      default: fused_group_sweep<2>(tile, tsize, gidx[g], gsrt[g], sg, st); break;
     }
-    dep[part][x] = d;
-  }
-  __syncthreads();
-  const uint32_t tsize = 1u << T;
-  const uint64_t ntiles = 1ull << (n - T);
-  for (uint64_t tl = blockIdx.x; tl < ntiles; tl += gridDim.x) {
-    uint64_t gbase = tl;
-    for (int k = 0; k < T; ++k) gbase = insert_zero(gbase, sq[k]);
-#pragma unroll 16
-    for (uint32_t i = threadIdx.x; i < tsize; i += blockDim.x) tile[i] = s[gbase | dep[0][i & 63] | dep[1][i >> 6]];
-    __syncthreads();
-    for (int g = 0; g < s_ngroups; ++g) {
-      switch (gsize[g]) {
-        case 1: fused_group_sweep<1>(tile, tsize, gidx[g], gsrt[g], sg, spos); break;
-        default: fused_group_sweep<2>(tile, tsize, gidx[g], gsrt[g], sg, spos); break;
-      }
-      __syncthreads();
-    }
-#pragma unroll 8
-    for (uint32_t i = threadIdx.x; i < tsize; i += blockDim.x) s[gbase | dep[0][i & 63] | dep[1][i >> 6]] = tile[i];
     __syncthreads();
   }
+#pragma unroll 4
+  for (uint32_t i = threadIdx.x; i < tsize; i += kFusedThreads) s[i] = tile[i];
 }
 
 // The same for states of 12 qubits and more: groups of four gates on distinct
