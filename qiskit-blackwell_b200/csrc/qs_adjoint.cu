@@ -221,7 +221,7 @@ struct PassArg {
   int32_t S[kAdjTileBits];  // tile positions (global qubits), ascending
   int32_t T, bits;    // tile bits, and those of them that exist (n < T)
   int32_t gb, ge;     // steps of the pass
-  int32_t slot0, nslots;  // first sum of the pass's part of the sweep, and how many it has
+  int32_t nslots;     // sums of the pass's part of the sweep
   int32_t from_zero;  // forward: the tile starts as |0..0> instead of being loaded
 };
 
@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(kThreads, FWD ? 3 : 2)
       double t = 0.0;
 #pragma unroll
       for (int w = 0; w < kThreads / 32; ++w) t += red[cur][w][tid];
-      partial[((uint64_t)b * P.nslots + G.slot[tid / 3] - P.slot0 + tid % 3) * ntiles + tile] = t;
+      partial[((uint64_t)b * P.nslots + G.slot[tid / 3] + tid % 3) * ntiles + tile] = t;
     }
     __syncwarp();   // the step is read above and its buffer refilled by this warp
   }
@@ -817,7 +817,7 @@ struct AdjPlan {
     for (int j = 0; j < T; ++j) col[j] = tile_col(j);
     cst = 0;
     out.clear();
-    P.slot0 = nslots;
+    const int slot0 = nslots;
     P.gb = (int)steps.size();
     for (size_t at = 0; at < cur.size(); ++at) {
       const int i = cur[at];
@@ -871,7 +871,7 @@ struct AdjPlan {
     if (count) block(which, count);
     steps.push_back(step(AG_STORE));
     P.ge = (int)steps.size();
-    P.nslots = nslots - P.slot0;
+    P.nslots = nslots - slot0;
     passes.push_back(P);
   }
 
@@ -1001,18 +1001,18 @@ extern "C" int qs_adjoint_gradient(qs_handle_t h, int n, const qs_op* ops, int n
     plan.sweep(order, true, rpasses);
     fpasses[0].from_zero = 1;
     const size_t most = std::max<size_t>(3, kAdjPartials / (sizeof(double) * nb * ntiles));
+    int32_t slot0 = 0;
     for (size_t k = 0; k < rpasses.size(); ++k) {
       const PassArg& P = rpasses[k];
-      if (parts.empty() || (size_t)(parts.back().nslots + P.nslots) > most) parts.push_back({k, k, P.slot0, 0});
+      if (parts.empty()) parts.push_back({0, 0, 0, 0});
+      else if ((size_t)(parts.back().nslots + P.nslots) > most) parts.push_back({k, k, slot0, 0});
       parts.back().pass1 = k + 1;
       parts.back().nslots += P.nslots;
+      slot0 += P.nslots;
     }
     for (const AdjPart& A : parts) {
       part_slots = std::max(part_slots, (size_t)A.nslots);
-      for (size_t k = A.pass0; k < A.pass1; ++k) {
-        rpasses[k].slot0 = A.slot0;
-        rpasses[k].nslots = A.nslots;
-      }
+      for (size_t k = A.pass0; k < A.pass1; ++k) rpasses[k].nslots = A.nslots;
     }
   }
 
@@ -1148,9 +1148,11 @@ extern "C" int qs_adjoint_gradient(qs_handle_t h, int n, const qs_op* ops, int n
   // ---- reverse sweep
   if (use_passes) {
     for (size_t k = 0; k < parts.size(); ++k) {
+      // the steps number the sums over all parts: the part's first is at the buffer's start
+      double* part0 = reinterpret_cast<double*>((uintptr_t)d_parts - sizeof(double) * ntiles * parts[k].slot0);
       for (size_t q = parts[k].pass0; q < parts[k].pass1; ++q) {
         k_adj_pass<false><<<dim3((unsigned)ntiles, nb), kThreads, pass_smem[1], h->stream>>>(
-            (float2*)work, vstride, rpasses[q], d_steps, d_mats, nb, d_u2, d_parts);
+            (float2*)work, vstride, rpasses[q], d_steps, d_mats, nb, d_u2, part0);
         qs_after_launch(h, "k_adj_pass");
       }
       if (parts[k].nslots > 0) {
