@@ -608,7 +608,7 @@ __device__ __forceinline__ void pauli_dot(const PauliMask<U>* __restrict__ sm, c
 }
 
 template <int M>
-constexpr uint32_t pauli_regs() { return M == 4 ? 0xC1u : M == 2 ? 0x41u : 0x01u; }
+constexpr uint32_t pauli_regs() { return M == 4 ? 0xC1u : 0x01u; }
 
 // The table of a Pauli sum, masks then terms, in shared memory.
 template <class U>
@@ -744,7 +744,7 @@ PauliUpload pauli_upload(qs_context* h, size_t offset, int n, const uint64_t* x,
       const uint64_t j = (uint64_t)(r & 1) | (((uint64_t)(r >> 1) << 6) ^ (x[k] & regs & ~1ull));
       pat |= (uint32_t)(__builtin_popcountll(j & z[k] & regs) & 1) << r;
     }
-    return pat & (regs == 0x01u ? 0x3u : regs == 0x41u ? 0xFu : 0xFFu);
+    return pat & (regs == 0x01u ? 0x3u : 0xFFu);
   };
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
     if (run_of(a) != run_of(b)) return run_of(a) < run_of(b);
