@@ -791,7 +791,9 @@ void pauli_apply(qs_context* h, const float2* in, float2* out, uint64_t vstride,
   const PauliUpload T = pauli_upload<U>(h, 0, n, x, z, c, nterms, pauli_regs<M>(), false);
   const uint64_t nthr = (1ull << n) / (2 * M), per = kThreads / S;
   if (T.bytes > 32 * 1024) qs_smem_limit(h, (const void*)k_pauli_apply<M, S, U>, pauli_largest<U>());
-  qs_launch_pdl(h, k_pauli_apply<M, S, U>, dim3((unsigned)((nthr + per - 1) / per), nb), dim3(kThreads), T.bytes, in, out,
+  // a CTA holds one vector: no more threads than that has work for
+  const unsigned threads = S == 1 ? (unsigned)std::min<uint64_t>(nthr, kThreads) : kThreads;
+  qs_launch_pdl(h, k_pauli_apply<M, S, U>, dim3((unsigned)((nthr + per - 1) / per), nb), dim3(threads), T.bytes, in, out,
                 vstride, T.table, T.runs, (U)nthr);
   qs_after_launch(h, "k_pauli_apply");
 }
@@ -802,11 +804,18 @@ void pauli_apply(qs_context* h, const float2* in, float2* out, uint64_t vstride,
 // apart; 16-byte aligned, not aliased.
 void qs_pauli_apply(qs_context* h, const float2* in, float2* out, uint64_t vstride, int nb, int n, const uint64_t* x,
                     const uint64_t* z, const double* c, int nterms) {
-  // Eight amplitudes per thread once they fill the SMs; below, two, and the
-  // masks over 8 groups of threads (shots and an expectation value of 64 terms:
-  // 82 us against 93 at 17 qubits, 94 against 92 at 18, 118 against 93 at 19).
+  // Eight amplitudes per thread, or two and the masks over 8 groups of threads:
+  // eight cost less in all, but a thread goes through every term (2.4 us + 0.26 per
+  // term while the SMs are not full), where two share the terms out and launch four
+  // times the threads for each of eight groups (2 us + (8 + 0.25 per term) for each
+  // 2^18 amplitudes).  Measured on both sides of the line, us for two / eight: 2^16
+  // amplitudes, 8 terms 4.5 / 4.7, 24 terms 6.3 / 8.4; 2^17 amplitudes, 24 terms 9.6 /
+  // 8.9, 64 terms 16 / 19; 15 vectors of 14 qubits, 64 terms 27 / 19; 1024 vectors of 8
+  // qubits, 64 terms 24.6 / 21.5 (40 in CTAs of 256 threads, of which 32 had work).
+  const double amps = std::ldexp((double)nb, n - 16);
+  const bool eight = n >= 8 && (amps >= 4.0 || nterms <= 8.0 * amps * amps);
   if (n > 32) pauli_apply<4, 1, uint64_t>(h, in, out, vstride, nb, n, x, z, c, nterms);
-  else if (n >= 8 && ((uint64_t)nb << n) >= (1ull << 18)) pauli_apply<4, 1, uint32_t>(h, in, out, vstride, nb, n, x, z, c, nterms);
+  else if (eight) pauli_apply<4, 1, uint32_t>(h, in, out, vstride, nb, n, x, z, c, nterms);
   else pauli_apply<1, 8, uint32_t>(h, in, out, vstride, nb, n, x, z, c, nterms);
 }
 
@@ -936,6 +945,9 @@ int qs_expect_pauli_sum(qs_handle_t h, const void* state, int n, const uint64_t*
   qs_check_state(state, n);
   QS_CHECK_ARG(out != nullptr, "out is null");
   QS_CHECK_ARG(nterms >= 1 && nterms <= 1024, "n_terms must be in [1, 1024]");
+  // as qs_pauli_apply; one vector fills the SMs from 18 qubits on (shots and an
+  // expectation value of 64 terms, two against eight amplitudes per thread: 82 us /
+  // 93 at 17 qubits, 94 / 92 at 18, 118 / 93 at 19)
   if (n > 32) pauli_expect<4, 1, uint64_t>(h, (const float2*)state, n, x, z, c, nterms);
   else if (n >= 18) pauli_expect<4, 1, uint32_t>(h, (const float2*)state, n, x, z, c, nterms);
   else pauli_expect<1, 8, uint32_t>(h, (const float2*)state, n, x, z, c, nterms);
