@@ -243,17 +243,20 @@ __global__ void __launch_bounds__(kFusedThreads, 2) k_fused1q_dev(float2* __rest
   for (uint32_t i = threadIdx.x; i < tsize; i += kFusedThreads) s[i] = tile[i];
 }
 
-// The same for states of 12 qubits and more: groups of four gates on distinct
-// tile positions, a thread holding the 16 amplitudes that a group mixes; byte
-// addresses built from the columns of the tile's bits; the next tile's 16-byte
-// copies (qubit 0 is in the tile unless twelve other qubits are targets) in
-// flight while one is worked on.
+// The same for states of 12 qubits and more: groups of four tile positions, a thread
+// holding the 16 amplitudes that a group mixes and applying all gates of each
+// position in their order; byte addresses built from the columns of the tile's bits;
+// the next tile's 16-byte copies (qubit 0 is in the tile unless twelve other qubits
+// are targets) in flight while one is worked on.
 //
 // Bound by issue: ten gates are 80 FMAs per amplitude, 37 us of FP32 time at 24
 // qubits, as many shared-memory and address instructions, and 41 us of HBM
 // beside them: 115-133 us; 187-202 in sweeps of two gates, which move the tile
 // five times through shared memory.  Three CTAs per SM spill (120 us, and 18.5
 // instead of 14.2 at 20 qubits); registers instead of cp.async cost the same.
+// Twelve gates on one qubit of 16: 10.7 us a call; 26 with a group for each.  The loop
+// over a position's gates only where a target repeats: run always, it costs eight
+// gates on 22 qubits 33.7 us instead of 29.8.
 constexpr int kTileThreads = 256;
 
 // The tile's columns: as tile_col, but bit 0 stays with position 0, so that a
@@ -270,7 +273,7 @@ __device__ __forceinline__ void copy_async8(uint32_t dst, const void* src) {
 
 struct FusedGroup {
   uint16_t v[4], rem[8];   // byte columns of the register bits and of the thread index
-  int32_t gate[4];         // gate on each register bit, -1 for none
+  int32_t gate[4];         // first gate on each register bit, -1 for none
 };
 
 __global__ void __launch_bounds__(kTileThreads, 2)
@@ -280,11 +283,14 @@ __global__ void __launch_bounds__(kTileThreads, 2)
   constexpr int T = kFusedMax;
   extern __shared__ __align__(16) unsigned char tile_smem[];
   __shared__ __align__(16) G2 sg[kFusedMax];
-  __shared__ FusedGroup grp[kFusedMax];
+  __shared__ FusedGroup grp[kFusedMax / 4];
+  __shared__ int nxt[kFusedMax];            // the next gate on the same target, -1 for none
+  __shared__ int last[T];                   // setup: the last gate so far on a position
   __shared__ int st[kFusedMax], sq[T];
   __shared__ uint64_t dep_lo[64], dep_hi[32];   // state index of a pair of amplitudes (tile bits 1-6, 7-11)
   __shared__ uint16_t map_lo[64], map_hi[32];   // its byte address in the tile
   __shared__ int s_groups;
+  __shared__ bool s_more;                   // some target has several gates
   const int tid = threadIdx.x;
   if (tid < K) st[tid] = targets[tid];
   if (tid < 4 * K) sg[tid >> 2].g[tid & 3] = gates[tid];
@@ -304,26 +310,34 @@ __global__ void __launch_bounds__(kTileThreads, 2)
       else m |= 1ull << st[k];
     }
     int ng = ok ? 0 : -1;
+    const bool more = __popcll(m) < K;
     if (ok) {
       for (int q = 0; __popcll(m) < T; ++q) m |= 1ull << q;
       uint64_t r = m;
       for (int j = 0; j < T; ++j, r &= r - 1) sq[j] = __ffsll((long long)r) - 1;
-      // a gate joins the group unless it is full or an earlier gate that is
-      // not done has its position
-      for (uint32_t done = 0; done != (1u << K) - 1u; ++ng) {
+      // positions in the order of their first gates, four to a group; a
+      // position's further gates follow by nxt
+      uint32_t seen = 0;
+      for (int k = 0; k < K; ++ng) {
         FusedGroup& G = grp[ng];
-        uint32_t seen = 0, bits = 0;
+        uint32_t bits = 0;
         int cnt = 0;
-        for (int k = 0; k < K; ++k) {
-          if ((done >> k) & 1) continue;
+        for (; k < K; ++k) {
           const int p = __popcll(m & ((1ull << st[k]) - 1ull));
-          if (cnt < 4 && !((seen >> p) & 1)) {
+          const bool first = !((seen >> p) & 1);
+          if (first && cnt == 4) break;
+          if (first) {
             G.gate[cnt] = k;
             G.v[cnt++] = (uint16_t)(pair_col(p) * 8);
             bits |= 1u << p;
-            done |= 1u << k;
+            seen |= 1u << p;
+          } else {
+            nxt[last[p]] = k;
           }
-          seen |= 1u << p;
+          if (more) {
+            nxt[k] = -1;
+            last[p] = k;
+          }
         }
         for (int p = T - 1; cnt < 4; --p)
           if (!((bits >> p) & 1)) {
@@ -338,9 +352,11 @@ __global__ void __launch_bounds__(kTileThreads, 2)
       atomicOr(status, 16u);
     }
     s_groups = ng;
+    s_more = more;
   }
   __syncthreads();
   const int ngroups = s_groups;
+  const bool more = s_more;
   if (ngroups < 0) return;
   const bool pairs = sq[0] == 0;
   if (tid < 96) {
@@ -395,10 +411,17 @@ __global__ void __launch_bounds__(kTileThreads, 2)
 #pragma unroll
       for (int r = 0; r < 16; ++r) w[r] = el(at[r]);
       const float4* U = reinterpret_cast<const float4*>(sg);
-      if (G.gate[0] >= 0) gate_on_bit<0>(w, U + 2 * G.gate[0]);
-      if (G.gate[1] >= 0) gate_on_bit<1>(w, U + 2 * G.gate[1]);
-      if (G.gate[2] >= 0) gate_on_bit<2>(w, U + 2 * G.gate[2]);
-      if (G.gate[3] >= 0) gate_on_bit<3>(w, U + 2 * G.gate[3]);
+      if (!more) {
+        if (G.gate[0] >= 0) gate_on_bit<0>(w, U + 2 * G.gate[0]);
+        if (G.gate[1] >= 0) gate_on_bit<1>(w, U + 2 * G.gate[1]);
+        if (G.gate[2] >= 0) gate_on_bit<2>(w, U + 2 * G.gate[2]);
+        if (G.gate[3] >= 0) gate_on_bit<3>(w, U + 2 * G.gate[3]);
+      } else {
+        for (int k = G.gate[0]; k >= 0; k = nxt[k]) gate_on_bit<0>(w, U + 2 * k);
+        for (int k = G.gate[1]; k >= 0; k = nxt[k]) gate_on_bit<1>(w, U + 2 * k);
+        for (int k = G.gate[2]; k >= 0; k = nxt[k]) gate_on_bit<2>(w, U + 2 * k);
+        for (int k = G.gate[3]; k >= 0; k = nxt[k]) gate_on_bit<3>(w, U + 2 * k);
+      }
 #pragma unroll
       for (int r = 0; r < 16; ++r) el(at[r]) = w[r];
       __syncthreads();
