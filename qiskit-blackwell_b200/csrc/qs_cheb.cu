@@ -1,7 +1,7 @@
 // qs_cheb.cu — CSR SpMV and the Chebyshev recurrence for exp(-iHt)|psi>.
 //
 // Rows are processed by V-lane sub-warps (V = 1..32, picked from the mean row
-// length and the number of rows).  A 20-qubit Hamiltonian of 30 entries per row
+// length and the number of rows; rows far above the mean by whole warps).  A 20-qubit Hamiltonian of 30 entries per row
 // takes 104 us per degree with V = 4 (4.3 TB/s of its 12 nnz + 44 N bytes) and
 // 322 us with a warp per row, whose gathers used 8 bytes of each 32-byte sector
 // and whose merge cost 150 instructions per row.  Each lane
@@ -366,7 +366,7 @@ __device__ __forceinline__ void pauli_run(const PMask* __restrict__ sp, int b, i
 //
 // Bound by the gathers' L2 traffic and their issue slots.  22 qubits, 42 masks:
 // 73 us per degree; 176 us with one amplitude per thread, of which the two
-// POPCs of a pair (16 lanes per clock and SM) alone are 137.
+// POPCs of a pair (16 lanes per clock and SM: 149 thousand cycles) alone are 78.
 template <int M, int S, bool FIRST>
 __global__ void __launch_bounds__(kPauliThreads)
     k_chebp_masks(const PMask* __restrict__ masks, PRuns R, uint32_t nthr, const float2* __restrict__ D,

@@ -21,7 +21,9 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kMaxBlocks = 1024;
-constexpr int kPauliBlocks = 888;   // 148 SMs x 2 resident CTAs x 3
+// Two waves of the three CTAs that fit on each of 148 SMs; a constant, so that the
+// order of an expectation value's sums depends on the width alone.
+constexpr int kPauliBlocks = 888;
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
